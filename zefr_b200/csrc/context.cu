@@ -18,67 +18,172 @@ using dev::TW;
 // layout conversion kernels
 // ---------------------------------------------------------------------------
 
+// State import and export move 8 + sizeof(T) bytes per value and compute
+// nothing, so they are bound by HBM as long as the index arithmetic stays off
+// the path: a thread owns one element and kRowsPerThread consecutive (point,
+// variable) rows, issues all of its loads before its stores, and finds a row's
+// point with a division by the compile-time variable count.  A warp reads 32
+// consecutive elements of a row (256 bytes for es = 1) and writes four tiles'
+// 8-element runs; the thread's rows are consecutive in the tile, so lines
+// fill up in L2.  TGV 64^3 P3 FP64 (671 MB each way), kernel alone: one value
+// per thread with four 64-bit divisions 474 us in, 426 us out; this form
+// 212 us in and 203 us out.
+constexpr int kRowsPerThread = 8, kConvThreads = 128;
+
 // reference-strided FP64 -> tile-major T, minus the reference state ref[v]
 // (nullptr: none); padded elements copy element 0
-template <typename T>
-__global__ void k_to_tiles(const double *__restrict__ src, T *__restrict__ dst, T *__restrict__ comp,
-                           const double *__restrict__ ref, int64_t neles, int64_t ntiles, int npts, int nv, int64_t ss,
-                           int64_t vs, int64_t es)
+template <typename T, int NV>
+__global__ void __launch_bounds__(kConvThreads)
+    k_to_tiles(const double *__restrict__ src, T *__restrict__ dst, T *__restrict__ comp,
+               const double *__restrict__ ref, int64_t neles, int64_t ntiles, int nrows, int64_t ss, int64_t vs,
+               int64_t es)
 {
-  const int64_t total = ntiles * npts * nv * TW;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
+  const int64_t i = (int64_t)blockIdx.x * kConvThreads + threadIdx.x;  // tile * TW + lane
+  if (i >= ntiles * TW) return;
+  const double *in = src + (i < neles ? i : 0) * es;
+  const int r0 = blockIdx.y * kRowsPerThread;
+  double x[kRowsPerThread];
+#pragma unroll
+  for (int k = 0; k < kRowsPerThread; k++)
   {
-    const int l = (int)(i % TW);
-    const int v = (int)((i / TW) % nv);
-    const int p = (int)((i / ((int64_t)TW * nv)) % npts);
-    const int64_t t = i / ((int64_t)TW * nv * npts);
-    int64_t e = t * TW + l;
-    if (e >= neles) e = 0;
-    const double x = src[p * ss + v * vs + e * es];
-    dst[i] = (T)(ref ? x - ref[v] : x);
-    if (comp) comp[i] = T(0);
+    const int r = r0 + k, p = r / NV, v = r % NV;
+    if (r < nrows) x[k] = in[p * ss + v * vs];
+  }
+  const int64_t o = ((i / TW) * nrows + r0) * TW + i % TW;
+#pragma unroll
+  for (int k = 0; k < kRowsPerThread; k++)
+    if (r0 + k < nrows)
+    {
+      dst[o + k * TW] = (T)(ref ? x[k] - ref[(r0 + k) % NV] : x[k]);
+      if (comp) comp[o + k * TW] = T(0);
+    }
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(kConvThreads)
+    k_from_tiles(const T *__restrict__ srcT, const T *__restrict__ comp, const double *__restrict__ ref,
+                 double *__restrict__ dst, int64_t neles, int nrows, int64_t ss, int64_t vs, int64_t es)
+{
+  const int64_t e = (int64_t)blockIdx.x * kConvThreads + threadIdx.x;
+  if (e >= neles) return;
+  const int r0 = blockIdx.y * kRowsPerThread;
+  const int64_t j = ((e / TW) * nrows + r0) * TW + e % TW;
+  T x[kRowsPerThread], c[kRowsPerThread];
+#pragma unroll
+  for (int k = 0; k < kRowsPerThread; k++)
+    if (r0 + k < nrows)
+    {
+      x[k] = srcT[j + k * TW];
+      c[k] = comp ? comp[j + k * TW] : T(0);
+    }
+#pragma unroll
+  for (int k = 0; k < kRowsPerThread; k++)
+  {
+    const int r = r0 + k, p = r / NV, v = r % NV;
+    if (r < nrows)
+    {
+      double val = (double)x[k];
+      if (comp) val -= (double)c[k];
+      if (ref) val += ref[v];
+      dst[e * es + p * ss + v * vs] = val;
+    }
   }
 }
 
-template <typename T>
-__global__ void k_from_tiles(const T *__restrict__ srcT, const T *__restrict__ comp, const double *__restrict__ ref,
-                             double *__restrict__ dst, int64_t neles, int npts, int nv, int64_t ss, int64_t vs,
-                             int64_t es)
+static dim3 conv_grid(int64_t n, int nrows)
 {
-  const int64_t total = neles * npts * nv;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
-  {
-    const int64_t e = i % neles;
-    const int v = (int)((i / neles) % nv);
-    const int p = (int)(i / (neles * nv));
-    const int64_t t = e / TW;
-    const int l = (int)(e % TW);
-    const int64_t j = ((t * npts + p) * nv + v) * TW + l;
-    double val = (double)srcT[j];
-    if (comp) val -= (double)comp[j];
-    if (ref) val += ref[v];
-    dst[p * ss + v * vs + e * es] = val;
-  }
+  return dim3((unsigned)((n + kConvThreads - 1) / kConvThreads),
+              (unsigned)((nrows + kRowsPerThread - 1) / kRowsPerThread));
 }
 
-// per-variable sum over all points and elements of a reference-strided array
-__global__ void k_var_sums(const double *__restrict__ src, int64_t neles, int npts, int nv, int64_t ss, int64_t vs,
-                           int64_t es, double *out)
+// state (strides ss, vs, es, on the device) -> tile layout
+template <typename T>
+static void to_tiles(Ctx *c, const double *src, T *dst, T *comp, const double *ref, int64_t ss, int64_t vs, int64_t es)
 {
-  double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  const int64_t n = neles * npts;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-  {
-    const int64_t e = i % neles;
-    const int p = (int)(i / neles);
-    for (int v = 0; v < nv; v++) acc[v] += src[p * ss + v * vs + e * es];
-  }
-  for (int v = 0; v < nv; v++)
+  ProfScope ps(*c, ZB_K_TO_TILES);
+  const int nrows = c->S * c->V;
+  const dim3 grid = conv_grid(c->ntiles * TW, nrows);
+  if (c->V == 4)
+    k_to_tiles<T, 4><<<grid, kConvThreads, 0, c->stream>>>(src, dst, comp, ref, c->plan.neles, c->ntiles, nrows, ss,
+                                                           vs, es);
+  else
+    k_to_tiles<T, 5><<<grid, kConvThreads, 0, c->stream>>>(src, dst, comp, ref, c->plan.neles, c->ntiles, nrows, ss,
+                                                           vs, es);
+  c->launches++;
+  CK(cudaGetLastError());
+}
+
+// Mean of every variable over all points and elements of a reference-strided
+// array, rounded to FP32 (0 where it is not finite): the mixed form's
+// reference state, into dref (device) and href (mapped host memory).  A block
+// sums kMeanPoints points of a stride of elements with all of their loads in
+// flight; block sums go to `partial` and the block that finishes last adds
+// them in block order, so the mean does not depend on the schedule.  One FP64
+// atomic per warp and variable to five addresses, which this replaces,
+// serialised: 470 us for 40^3 P3 hexahedra (164 MB), now 54 us.
+constexpr int kMeanThreads = 256, kMeanPoints = 4, kMeanBlocks = 148 * 4;
+
+template <int NV>
+__global__ void __launch_bounds__(kMeanThreads)
+    k_state_mean(const double *__restrict__ src, int64_t neles, int npts, int64_t ss, int64_t vs, int64_t es,
+                 double *partial, unsigned *done, double *dref, volatile double *href)
+{
+  __shared__ double red[NV][kMeanThreads / 32];
+  __shared__ bool last;
+  double acc[NV];
+#pragma unroll
+  for (int v = 0; v < NV; v++) acc[v] = 0.0;
+  for (int p0 = blockIdx.y * kMeanPoints; p0 < npts; p0 += gridDim.y * kMeanPoints)
+    for (int64_t e = (int64_t)blockIdx.x * kMeanThreads + threadIdx.x; e < neles;
+         e += (int64_t)gridDim.x * kMeanThreads)
+    {
+      double x[kMeanPoints][NV];
+#pragma unroll
+      for (int k = 0; k < kMeanPoints; k++)
+#pragma unroll
+        for (int v = 0; v < NV; v++) x[k][v] = p0 + k < npts ? src[(p0 + k) * ss + v * vs + e * es] : 0.0;
+#pragma unroll
+      for (int v = 0; v < NV; v++)
+#pragma unroll
+        for (int k = 0; k < kMeanPoints; k++) acc[v] += x[k][v];
+    }
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+#pragma unroll
+  for (int v = 0; v < NV; v++)
   {
     double x = acc[v];
     for (int o = 16; o > 0; o /= 2) x += __shfl_down_sync(0xffffffff, x, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&out[v], x);
+    if (lane == 0) red[v][warp] = x;
   }
+  __syncthreads();
+  const int nblocks = gridDim.x * gridDim.y, block = blockIdx.y * gridDim.x + blockIdx.x;
+  if (threadIdx.x < NV)
+  {
+    double x = 0.0;
+    for (int w = 0; w < kMeanThreads / 32; w++) x += red[threadIdx.x][w];
+    partial[block * NV + threadIdx.x] = x;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == (unsigned)nblocks - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (warp < NV)
+  {
+    double x = 0.0;
+    for (int b = lane; b < nblocks; b += 32) x += __ldcg(partial + b * NV + warp);
+    for (int o = 16; o > 0; o /= 2) x += __shfl_down_sync(0xffffffff, x, o);
+    if (lane == 0)
+    {
+      const double mean = x / ((double)neles * npts);
+      const double ur = isfinite(mean) ? (double)(float)mean : 0.0;
+      dref[warp] = ur;
+      href[warp] = ur;
+    }
+  }
+  if (threadIdx.x == 0) *done = 0;
+  __threadfence_system();
 }
 
 // FP64 residual norms of report_residuals: max, sum |r|, sum r^2 with r = divF/|J|
@@ -345,7 +450,7 @@ static void launch_stage_impl(Ctx &c, const StageCfg &sc)
       const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(A);
       set_smem(dev::k_hex_euler<T, A, N>, smem);
       ProfScope ps(c, ZB_K_EULER);
-      dev::k_hex_euler<T, A, N><<<(unsigned)c.ntiles, HT, smem, c.stream>>>(a, ops);
+      dev::k_hex_euler<T, A, N><<<(unsigned)c.ntiles, HT * dev::HexEulerShape<A, N>::zs, smem, c.stream>>>(a, ops);
       c.launches++;
       CK(cudaGetLastError());
     }
@@ -536,10 +641,12 @@ static void free_all(Ctx *c)
                   c->Ufp[1], c->Fvn, c->Fcom, c->mets, c->fgeo, c->Ucomp, c->nbr, c->dtmp, c->dred, c->dref,
                   c->dU, c->dweights, c->dfun, c->lam, c->Lfp, c->Ubfp, c->dUbfp, c->UCb, c->Ubx, c->Ubar, c->pbar, c->dops, c->dwall,
                   c->mbar, c->gbar, c->nbx, c->mbar_acc, c->gbar_acc, c->d_dt, c->dt_ele, c->h_ref, c->evol,
-                  c->dfw, c->U_til, c->rk_err, c->rkv, c->rkfvn, c->geo_tab, c->geo_pair, c->geo_work};
+                  c->dfw, c->U_til, c->rk_err, c->rkv, c->rkfvn, c->geo_tab, c->geo_pair, c->geo_work, c->dmean};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (c->tc_err_host) cudaFreeHost(const_cast<int *>(c->tc_err_host));
+  if (c->mean_host) cudaFreeHost(c->mean_host);
+  if (c->mean_ready) cudaEventDestroy(c->mean_ready);
   for (int b = 0; b < 2; b++)
   {
     if (c->pipe_in[b]) cudaFree(c->pipe_in[b]);
@@ -675,6 +782,15 @@ Ctx *ctx_create(const Plan &plan)
       c->tc_err_dev = static_cast<int *>(dp);
     }
     CK(cudaMemsetAsync(c->dref, 0, 8 * sizeof(double), c->stream));
+    if (c->prec != ZB_FP64)
+    {
+      // reference-state reduction: block sums and arrival counter, the result
+      // for the host and the event that says it is there
+      c->dmean = (double *)dalloc((kMeanBlocks * 5 + 1) * sizeof(double));
+      CK(cudaMemsetAsync(c->dmean, 0, (kMeanBlocks * 5 + 1) * sizeof(double), c->stream));
+      CK(cudaHostAlloc((void **)&c->mean_host, 8 * sizeof(double), cudaHostAllocMapped));
+      CK(cudaEventCreateWithFlags(&c->mean_ready, cudaEventDisableTiming));
+    }
     if (c->prec == ZB_FP64)
       upload_static<double>(*c);
     else
@@ -781,36 +897,31 @@ void ctx_set_state(Ctx *c, const double *U, int64_t ss, int64_t vs, int64_t es, 
   if (!U) ZB_THROW(ZB_ERR_ARG, "null state");
   const size_t ext = extent(c, ss, vs, es, c->S);
   const double *src = stage_in(c, U, ext, where);
-  const int64_t work = c->ntiles * c->S * c->V * TW;
-  if (c->prec != ZB_FP64)
+  if (c->prec == ZB_FP64)
+    to_tiles<double>(c, src, (double *)c->U, nullptr, nullptr, ss, vs, es);
+  else
   {
     // reference state of the perturbation form: the state's mean per variable
-    // (FP64 reduction), rounded to FP32 so U = Ur + U' holds exactly in FP32
-    CK(cudaMemsetAsync(c->dred, 0, 8 * sizeof(double), c->stream));
-    const int64_t n = c->plan.neles * c->S;
-    k_var_sums<<<grid_for(n, 256), 256, 0, c->stream>>>(src, c->plan.neles, c->S, c->V, ss, vs, es, c->dred);
-    c->launches++;
-    CK(cudaGetLastError());
-    double h[8];
-    CK(cudaMemcpyAsync(h, c->dred, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    for (int v = 0; v < c->V; v++)
-    {
-      const double mean = h[v] / (double)n;
-      c->uref[v] = std::isfinite(mean) ? (double)(float)mean : 0.0;
-    }
-    CK(cudaMemcpyAsync(c->dref, c->uref, sizeof(c->uref), cudaMemcpyHostToDevice, c->stream));
-  }
-  {
-    ProfScope ps(*c, ZB_K_TO_TILES);
-    if (c->prec == ZB_FP64)
-      k_to_tiles<double><<<grid_for(work, 256), 256, 0, c->stream>>>(src, (double *)c->U, nullptr, nullptr,
-                                                                       c->plan.neles, c->ntiles, c->S, c->V, ss, vs, es);
+    // (FP64 reduction), rounded to FP32 so U = Ur + U' holds exactly in FP32.
+    // The conversion reads it on the device; the host, whose later launches
+    // pass it by value, waits for the reduction while the conversion runs.
+    const int64_t E = c->plan.neles;
+    const int64_t ye = (c->S + kMeanPoints - 1) / kMeanPoints;
+    const int64_t xe = std::max<int64_t>(1, std::min((E + kMeanThreads - 1) / kMeanThreads, kMeanBlocks / ye));
+    const dim3 grid((unsigned)xe, (unsigned)ye);
+    double *href = nullptr;
+    CK(cudaHostGetDevicePointer((void **)&href, c->mean_host, 0));
+    unsigned *done = (unsigned *)(c->dmean + kMeanBlocks * 5);
+    if (c->V == 4)
+      k_state_mean<4><<<grid, kMeanThreads, 0, c->stream>>>(src, E, c->S, ss, vs, es, c->dmean, done, c->dref, href);
     else
-      k_to_tiles<float><<<grid_for(work, 256), 256, 0, c->stream>>>(src, (float *)c->U, (float *)c->Ucomp, c->dref,
-                                                                      c->plan.neles, c->ntiles, c->S, c->V, ss, vs, es);
+      k_state_mean<5><<<grid, kMeanThreads, 0, c->stream>>>(src, E, c->S, ss, vs, es, c->dmean, done, c->dref, href);
     c->launches++;
     CK(cudaGetLastError());
+    CK(cudaEventRecord(c->mean_ready, c->stream));
+    to_tiles<float>(c, src, (float *)c->U, (float *)c->Ucomp, c->dref, ss, vs, es);
+    CK(cudaEventSynchronize(c->mean_ready));
+    for (int v = 0; v < c->V; v++) c->uref[v] = c->mean_host[v];
   }
   if (where == ZB_HOST) CK(cudaStreamSynchronize(c->stream));
   c->ufp_valid = false;
@@ -837,17 +948,20 @@ static void from_tiles(Ctx *c, const void *srcT, const void *comp, const double 
     if (ext != (size_t)c->S * c->V * c->plan.neles)
       CK(cudaMemcpyAsync(dst, out, bytes, cudaMemcpyHostToDevice, c->stream));
   }
-  const int64_t work = c->plan.neles * c->S * c->V;
   {
-  ProfScope ps(*c, ZB_K_FROM_TILES);
-  if (c->prec == ZB_FP64)
-    k_from_tiles<double><<<grid_for(work, 256), 256, 0, c->stream>>>((const double *)srcT, (const double *)comp, ref,
-                                                                       dst, c->plan.neles, c->S, c->V, ss, vs, es);
-  else
-    k_from_tiles<float><<<grid_for(work, 256), 256, 0, c->stream>>>((const float *)srcT, (const float *)comp, ref,
-                                                                      dst, c->plan.neles, c->S, c->V, ss, vs, es);
-  c->launches++;
-  CK(cudaGetLastError());
+    ProfScope ps(*c, ZB_K_FROM_TILES);
+    const int64_t E = c->plan.neles;
+    const int nrows = c->S * c->V;
+    const dim3 grid = conv_grid(E, nrows);
+    auto launch = [&](auto kernel, auto *t, auto *r) {
+      kernel<<<grid, kConvThreads, 0, c->stream>>>(t, r, ref, dst, E, nrows, ss, vs, es);
+    };
+    if (c->prec == ZB_FP64)
+      launch(c->V == 4 ? k_from_tiles<double, 4> : k_from_tiles<double, 5>, (const double *)srcT, (const double *)comp);
+    else
+      launch(c->V == 4 ? k_from_tiles<float, 4> : k_from_tiles<float, 5>, (const float *)srcT, (const float *)comp);
+    c->launches++;
+    CK(cudaGetLastError());
   }
   if (where == ZB_HOST)
   {
@@ -1249,14 +1363,7 @@ void ctx_vjp(Ctx *c, const double *lam, double *Ubar, int64_t ss, int64_t vs, in
   if (!lam || !Ubar) ZB_THROW(ZB_ERR_ARG, "null adjoint buffer");
   const size_t ext = extent(c, ss, vs, es, c->S);
   const double *src = stage_in(c, lam, ext, where);
-  {
-    const int64_t work = c->ntiles * c->S * c->V * TW;
-    ProfScope ps(*c, ZB_K_TO_TILES);
-    k_to_tiles<double><<<grid_for(work, 256), 256, 0, c->stream>>>(src, c->lam, nullptr, nullptr, c->plan.neles,
-                                                                     c->ntiles, c->S, c->V, ss, vs, es);
-    c->launches++;
-    CK(cudaGetLastError());
-  }
+  to_tiles<double>(c, src, c->lam, nullptr, nullptr, ss, vs, es);
   vjp_tiles(c, param_bar != nullptr, param_bar, geo, accumulate);
   from_tiles(c, c->Ubar, nullptr, nullptr, Ubar, ss, vs, es, where);
   if (geo_out) geo_to_reference(c, c->mbar, c->gbar, inv_jaco_bar, jaco_det_bar, norm_bar, dA_bar);
@@ -1359,13 +1466,9 @@ void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar
   {
     const size_t ext = extent(c, ss, vs, es, c->S);
     const double *src = stage_in(c, U0, ext, where);
-    k_to_tiles<double><<<grid, 256, 0, c->stream>>>(src, Us[0], nullptr, nullptr, c->plan.neles, c->ntiles, S, V, ss,
-                                                    vs, es);
+    to_tiles<double>(c, src, Us[0], nullptr, nullptr, ss, vs, es);
     src = stage_in(c, Ubar1, ext, where);
-    k_to_tiles<double><<<grid, 256, 0, c->stream>>>(src, ub1, nullptr, nullptr, c->plan.neles, c->ntiles, S, V, ss,
-                                                    vs, es);
-    c->launches += 2;
-    CK(cudaGetLastError());
+    to_tiles<double>(c, src, ub1, nullptr, nullptr, ss, vs, es);
   }
   // forward: the stage states and residuals (FRSolver::step_RK's stages)
   for (int s = 0; s < 4; s++)

@@ -1,6 +1,7 @@
 // Device context shared by the forward (context.cu) and adjoint (adjoint.cu)
 // translation units: buffers, launch helpers and profiling scopes.
 #pragma once
+#include <algorithm>
 #include <cstring>
 #include <cmath>
 #include <mutex>
@@ -73,6 +74,9 @@ struct Ctx
   // deviates from; zero for the FP64 form
   double uref[5] = {0, 0, 0, 0, 0};
   double *dref = nullptr;  // device copy for the conversion kernels
+  // its reduction: block sums and counter, the host's copy (mapped), its event
+  double *dmean = nullptr, *mean_host = nullptr;
+  cudaEvent_t mean_ready = nullptr;
   void *dU = nullptr;          // physical gradient side output (functionals)
   double *dweights = nullptr;  // quadrature weights of the solution points
   double *dfun = nullptr;      // functional reduction buffer
