@@ -1,10 +1,8 @@
-// Device context: buffers in the tile-major layout, layout conversion, kernel
-// dispatch over (dimension, order, precision) and explicit RK44 stepping.
+// Device context: buffers in the tile-major layout, layout conversion,
+// reductions and explicit RK44 stepping.  The residual kernels are launched
+// from one translation unit per element type (quad_stage.cu, tri_stage.cu,
+// hex_stage_*.cu).
 #include "ctx_impl.cuh"
-#include "hex_kernels.cuh"
-#include "tri_kernels.cuh"
-#include "tri_tc_kernels.cuh"
-#include "time_kernels.cuh"
 
 namespace zb {
 
@@ -411,212 +409,22 @@ __global__ void k_wall_force(const T *__restrict__ Ufp, const T *__restrict__ dU
   }
 }
 
-// ---------------------------------------------------------------------------
-// dispatch
-// ---------------------------------------------------------------------------
-
-
-template <typename T, typename A, int D, int N>
-static void launch_extrap_impl(Ctx &c)
+// selects the forward kernels of the context's element type, order and form
+static void bind_forward(Ctx &c)
 {
-  using G = Shape<D, N>;
-  const int64_t work = c.ntiles * G::Fp * TW;
-  ProfScope ps(c, ZB_K_EXTRAP);
-  if constexpr (D == 3)
-    dev::k_hex_extrap<T, A, N><<<(unsigned)c.ntiles, TW * N * N, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur],
-                                                                                c.ntiles, line_ops<A, N>(c.plan));
-  else
-    dev::k_extrap<T, A, D, N><<<grid_for(work, 256), 256, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur],
-                                                                           c.ntiles, line_ops<A, N>(c.plan));
-  c.launches++;
-  CK(cudaGetLastError());
-}
-
-
-template <typename T, typename A, int D, int N>
-static void launch_stage_impl(Ctx &c, const StageCfg &sc)
-{
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, NT = G::NT;
-  const Args<T, A> a = make_args<T, A>(c, sc);
-  const LineOpsT<A, N> ops = line_ops<A, N>(c.plan);
-  const size_t ops_bytes = sizeof(LineOpsT<A, N>);
-  if constexpr (D == 3)
-  {
-    // hexahedra: column-mapped kernels, TW x N^2 threads per tile
-    constexpr int HT = TW * N * N;
-    if (!c.plan.params.viscous)
-    {
-      const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(A);
-      set_smem(dev::k_hex_euler<T, A, N>, smem);
-      ProfScope ps(c, ZB_K_EULER);
-      dev::k_hex_euler<T, A, N><<<(unsigned)c.ntiles, HT * dev::HexEulerShape<A, N>::zs, smem, c.stream>>>(a, ops);
-      c.launches++;
-      CK(cudaGetLastError());
-    }
-    else
-    {
-      constexpr int ZG = dev::HexNsShape<A, N>::grad_zs, ZF = dev::HexNsShape<A, N>::face_zs;
-      const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(A);  // + sX padding
-      set_smem(dev::k_hex_ns_grad<T, A, N>, smem1);
-      if (!sc.face_only)
-      {
-        ProfScope ps(c, ZB_K_NS_GRAD);
-        dev::k_hex_ns_grad<T, A, N><<<(unsigned)c.ntiles, HT * ZG, smem1, c.stream>>>(a, ops);
-        c.launches++;
-        CK(cudaGetLastError());
-      }
-      if (sc.grad_only) return;
-      const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A);
-      set_smem(dev::k_hex_ns_face<T, A, N>, smem2);
-      ProfScope ps(c, ZB_K_NS_FACE);
-      dev::k_hex_ns_face<T, A, N><<<(unsigned)c.ntiles, HT * ZF, smem2, c.stream>>>(a, ops);
-      c.launches++;
-      CK(cudaGetLastError());
-    }
-    if (sc.extrap_next)
-    {
-      if (a.Fcom)
-        c.ufp_valid = false;  // the state changed and no traces were stored
-      else
-        c.cur ^= 1;
-    }
-    return;
-  }
-  if (!c.plan.params.viscous)
-  {
-    const size_t smem = (size_t)(S * V + D * S * V + Fp * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_euler<T, A, D, N>, smem);
-    ProfScope ps(c, ZB_K_EULER);
-    dev::k_euler<T, A, D, N><<<(unsigned)c.ntiles, NT, smem, c.stream>>>(a, ops);
-    c.launches++;
-    CK(cudaGetLastError());
-  }
-  else
-  {
-    const size_t smem1 = (size_t)(S * V + Fp * V + D * S * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_ns_grad<T, A, D, N>, smem1);
-    if (!sc.face_only)
-    {
-      ProfScope ps(c, ZB_K_NS_GRAD);
-      dev::k_ns_grad<T, A, D, N><<<(unsigned)c.ntiles, NT, smem1, c.stream>>>(a, ops);
-      c.launches++;
-      CK(cudaGetLastError());
-    }
-    if (sc.grad_only) return;
-    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_ns_face<T, A, D, N>, smem2);
-    ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_ns_face<T, A, D, N><<<(unsigned)c.ntiles, NT, smem2, c.stream>>>(a, ops);
-    c.launches++;
-    CK(cudaGetLastError());
-  }
-  if (sc.extrap_next) c.cur ^= 1;
-}
-
-
-// Triangles: dense-operator kernels (tri_kernels.cuh)
-template <typename T, typename A, int N>
-static void launch_extrap_tri(Ctx &c)
-{
-  using G = dev::TriShape<N>;
-  ProfScope ps(c, ZB_K_EXTRAP);
-  dev::k_tri_extrap<T, A, N><<<grid_for(c.ntiles * G::Fp * TW, 128), 128, 0, c.stream>>>(
-      (const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles, (const A *)c.dops);
-  c.launches++;
-  CK(cudaGetLastError());
-}
-
-template <typename T, typename A, int N>
-static void launch_stage_tri(Ctx &c, const StageCfg &sc)
-{
-  using G = dev::TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2;
-  const Args<T, A> a = make_args<T, A>(c, sc);
-  if (c.tc_err_host && *c.tc_err_host)
-  {
-    *c.tc_err_host = 0;
-    ZB_THROW(ZB_ERR_CUDA, "a tensor-core completion wait of an earlier launch timed out");
-  }
-  const size_t ops = (size_t)G::OPS_PAD;
-  if (!c.plan.params.viscous)
-  {
-    const size_t smem = (ops + (size_t)(S * V + D * S * V + Fp * V) * TW) * sizeof(A);
-    set_smem(dev::k_tri_euler<T, A, N>, smem);
-    ProfScope ps(c, ZB_K_EULER);
-    dev::k_tri_euler<T, A, N><<<(unsigned)c.ntiles, 128, smem, c.stream>>>(a);
-    c.launches++;
-    CK(cudaGetLastError());
-  }
-  else
-  {
-    const size_t smem1 = (ops + (size_t)(S * V + Fp * V + D * S * V) * TW) * sizeof(A);
-    if (!sc.face_only)
-    {
-      ProfScope ps(c, ZB_K_NS_GRAD);
-      bool launched = false;
-      if constexpr (std::is_same<A, float>::value && N <= 5)
-      {
-        if (c.plan.params.tensor_ops)
-        {
-          using C = dev::TriTc<N>;
-          set_smem(dev::k_tri_ns_grad_tc<N>, C::SMEM);
-          const int64_t groups = (c.ntiles + C::TILES - 1) / C::TILES;
-          dev::k_tri_ns_grad_tc<N><<<(unsigned)groups, C::NT, C::SMEM, c.stream>>>(a);
-          launched = true;
-        }
-      }
-      if (!launched)
-      {
-        set_smem(dev::k_tri_ns_grad<T, A, N>, smem1);
-        dev::k_tri_ns_grad<T, A, N><<<(unsigned)c.ntiles, 128, smem1, c.stream>>>(a);
-      }
-      c.launches++;
-      CK(cudaGetLastError());
-    }
-    if (sc.grad_only) return;
-    const size_t smem2 = (ops + (size_t)(Fp * V + S * V) * TW) * sizeof(A);
-    set_smem(dev::k_tri_ns_face<T, A, N>, smem2);
-    ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_tri_ns_face<T, A, N><<<(unsigned)c.ntiles, 128, smem2, c.stream>>>(a);
-    c.launches++;
-    CK(cudaGetLastError());
-  }
-  if (sc.extrap_next) c.cur ^= 1;
-}
-
-template <typename T, typename A, int D, int N>
-static void bind(Ctx &c)
-{
-  c.launch_extrap = &launch_extrap_impl<T, A, D, N>;
-  c.launch_stage = &launch_stage_impl<T, A, D, N>;
-  c.launch_dt = &launch_dt_impl<T, A, D, N>;
-}
-
-template <typename T, typename A>
-static void bind_t(Ctx &c)
-{
-  const int D = c.D, N = c.N;
   if (c.plan.etype == ET_TRI)
-  {
-#define ZB_BIND_TRI(NN)                                   \
-  if (N == NN)                                            \
-  {                                                       \
-    c.launch_extrap = &launch_extrap_tri<T, A, NN>;       \
-    c.launch_stage = &launch_stage_tri<T, A, NN>;         \
-    return;                                               \
-  }
-    ZB_BIND_TRI(2) ZB_BIND_TRI(3) ZB_BIND_TRI(4) ZB_BIND_TRI(5) ZB_BIND_TRI(6) ZB_BIND_TRI(7) ZB_BIND_TRI(8)
-    ZB_BIND_TRI(9)
-#undef ZB_BIND_TRI
-    ZB_THROW(ZB_ERR_UNSUPPORTED, "no triangle kernels for P=" + std::to_string(N - 1));
-  }
-#define ZB_BIND(DD, NN) \
-  if (D == DD && N == NN) { bind<T, A, DD, NN>(c); return; }
-  ZB_BIND(2, 2) ZB_BIND(2, 3) ZB_BIND(2, 4) ZB_BIND(2, 5) ZB_BIND(2, 6)
-  ZB_BIND(3, 2) ZB_BIND(3, 3) ZB_BIND(3, 4) ZB_BIND(3, 5)
-#undef ZB_BIND
-  ZB_THROW(ZB_ERR_UNSUPPORTED, "no kernels built for ndims=" + std::to_string(D) + " P=" + std::to_string(N - 1));
+    bind_tri(c);
+  else if (c.D == 2)
+    bind_quad(c);
+  else if (c.prec == ZB_FP64)
+    bind_hex_f64(c);
+  else
+    bind_hex_f32(c);
+  if (!c.launch_stage)
+    ZB_THROW(ZB_ERR_UNSUPPORTED,
+             c.plan.etype == ET_TRI
+                 ? "no triangle kernels for P=" + std::to_string(c.N - 1)
+                 : "no kernels built for ndims=" + std::to_string(c.D) + " P=" + std::to_string(c.N - 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -743,13 +551,8 @@ Ctx *ctx_create(const Plan &plan)
   if (plan.params.tensor_ops && !(c->prec == ZB_MIXED && plan.etype == ET_TRI && plan.params.viscous && plan.order <= 4))
     ZB_THROW(ZB_ERR_UNSUPPORTED, "tensor-core operator products are built for the mixed form on triangles "
                                  "(Navier-Stokes, P <= 4)");
-  if (c->prec == ZB_FP64)
-  {
-    bind_t<double, double>(*c);
-    bind_vjp(*c);
-  }
-  else
-    bind_t<float, float>(*c);
+  bind_forward(*c);
+  if (c->prec == ZB_FP64) bind_vjp(*c);
   try
   {
     const size_t nU = (size_t)c->ntiles * c->S * c->V * TW;

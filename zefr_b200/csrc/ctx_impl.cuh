@@ -283,6 +283,12 @@ static Args<T, A> make_args(Ctx &c, const StageCfg &sc)
   return a;
 }
 
+// select the forward kernels of the context's order (launch_extrap,
+// launch_stage, launch_dt; left null for an order not built)
+void bind_quad(Ctx &c);
+void bind_tri(Ctx &c);
+void bind_hex_f64(Ctx &c);
+void bind_hex_f32(Ctx &c);
 // selects the adjoint kernels of the context (plain FP64 form; adjoint.cu)
 void bind_vjp(Ctx &c);
 

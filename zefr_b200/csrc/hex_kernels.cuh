@@ -101,13 +101,27 @@ __device__ __forceinline__ bool q_minus(int q) { return (q & 1) == 0; }
 
 // k-th of the own flux points a thread handles when ZS threads share a column:
 // all six for ZS = 1; for ZS = 2 half 0 takes faces z-, x+, y- and half 1
-// takes z+, x-, y+, so the work done by only one side of a face (the LDG
-// normal flux, usually the side with the + face) is spread over both halves
+// takes z+, x-, y+; for ZS = 3 each third takes one axis' - and the next
+// axis' + face, so the work done by only one side of a face (the LDG normal
+// flux, usually the side with the + face) is spread over the threads
 template <int ZS>
 __device__ __forceinline__ int own_face(int zs, int k)
 {
-  return ZS == 1 ? k : 2 * k + ((zs + k) & 1);
+  if (ZS == 1) return k;
+  if (ZS == 2) return 2 * k + ((zs + k) & 1);
+  return k == 0 ? 2 * zs : (2 * zs + 3) % 6;
 }
+
+// z-levels of a column shared by ZS threads: thread zs takes levels
+// [zs * NZ, min(N, (zs + 1) * NZ))
+template <int N, int ZS>
+struct ZSplit
+{
+  static_assert(ZS >= 1 && ZS <= 3, "own_face deals the six flux points of a column to one, two or three threads");
+  static constexpr int NZ = (N + ZS - 1) / ZS;
+  static constexpr bool even = NZ * ZS == N;
+  static_assert(NZ * (ZS - 1) < N, "every thread of a column has a level");
+};
 
 template <typename T, typename A, int N>
 __device__ __forceinline__ void load_face_geo(const Args<T, A> &a, int64_t tile, int f, int l, A n[3], A &dA, int &code)
@@ -478,17 +492,39 @@ __device__ __forceinline__ void load_adj(const Args<T, A> &a, int64_t tile, int 
 // ---------------------------------------------------------------------------
 // Euler: volume flux, common flux, divergence (+RK, +next extrapolation)
 // ---------------------------------------------------------------------------
+// Launch shape of the Euler kernel: zs threads share a column, minb CTAs per
+// SM bound the registers.  One thread per column left 2-7 warps per CTA beside
+// 18-208 KB (FP64) of shared memory, too few to cover the metric and trace
+// loads; the split costs nothing but the barrier.  Timed on B200 (Rusanov,
+// jittered boxes, us per residual, zs = 1 -> this table): FP64 P1 40^3 77 ->
+// 66, P2 29^3 109 -> 88, P3 24^3 119 -> 87, P4 20^3 150 -> 117; mixed 44 ->
+// 41, 51 -> 43, 56 -> 47, 72 -> 60.  P2 with two threads per column or with
+// four CTAs per SM (72 registers, 400 bytes spilled) was no better than one.
+template <typename A, int N>
+struct HexEulerShape
+{
+  static constexpr bool f64 = sizeof(A) == 8;
+  static constexpr int zs = N == 3 ? 3 : 2;
+  static constexpr int minb = N == 2   ? (f64 ? 8 : 16)
+                              : N == 3 ? (f64 ? 3 : 5)
+                              : N == 4 ? (f64 ? 2 : 4)
+                                       : (f64 ? 1 : 2);
+};
+
 template <typename T, typename A, int N>
-__global__ void __launch_bounds__(TW * N * N) k_hex_euler(const __grid_constant__ Args<T, A> a,
-                                                          const __grid_constant__ LineOpsT<A, N> ops)
+__global__ void __launch_bounds__(TW * N * N * HexEulerShape<A, N>::zs, HexEulerShape<A, N>::minb)
+    k_hex_euler(const __grid_constant__ Args<T, A> a, const __grid_constant__ LineOpsT<A, N> ops)
 {
   using H = HexIdx<N>;
-  constexpr int S = H::S, V = 5;
+  constexpr int ZS = HexEulerShape<A, N>::zs;
+  using Z = ZSplit<N, ZS>;
+  constexpr int S = H::S, V = 5, NZ = Z::NZ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sU = reinterpret_cast<A *>(smem_raw);   // [S][V][TW] state, then new state
   A *sF = sU + S * V * TW;                   // [3][S][V][TW] transformed flux
   A *sFc = sF + 3 * S * V * TW;              // [Fp][V][TW]
-  const int l = threadIdx.x % TW, c = threadIdx.x / TW, ix = c % N, iy = c / N;
+  const int l = threadIdx.x % TW, c = (threadIdx.x / TW) % H::N2, zs = threadIdx.x / (TW * H::N2);
+  const int ix = c % N, iy = c / N, iz0 = zs * NZ, iz1 = Z::even ? iz0 + NZ : min(N, iz0 + NZ);
   const int64_t tile = blockIdx.x;
   if (tile >= a.ntiles) return;
   RowOps<A, N> o;
@@ -497,7 +533,7 @@ __global__ void __launch_bounds__(TW * N * N) k_hex_euler(const __grid_constant_
   H::fpts(ix, iy, f);
   const T *Ut = a.U + tile * (int64_t)S * V * TW;
 #pragma unroll 1
-  for (int iz = 0; iz < N; iz++)
+  for (int iz = iz0; iz < iz1; iz++)
   {
     const int s = ix + N * iy + H::N2 * iz;
     A U[V], F[V][3], P, Pp, adj[3][3], det;
@@ -516,10 +552,10 @@ __global__ void __launch_bounds__(TW * N * N) k_hex_euler(const __grid_constant_
         sF[((d1 * S + s) * V + v) * TW + l] = t;
       }
   }
-  hex_common_flux<T, A, N, false>(a, tile, l, ix, iy, sFc);
+  hex_common_flux<T, A, N, false, ZS>(a, tile, l, ix, iy, sFc, zs);
   __syncthreads();
 #pragma unroll 1
-  for (int iz = 0; iz < N; iz++)
+  for (int iz = iz0; iz < iz1; iz++)
   {
     const int s = ix + N * iy + H::N2 * iz;
     A res[V];
@@ -540,27 +576,35 @@ __global__ void __launch_bounds__(TW * N * N) k_hex_euler(const __grid_constant_
   if (a.extrap_next)
   {
     __syncthreads();
-    hex_extrap_next<T, A, N>(a, tile, l, ix, iy, f, sU, ops);
+    hex_extrap_next<T, A, N, ZS>(a, tile, l, ix, iy, f, sU, ops, zs);
   }
 }
 
 // ---------------------------------------------------------------------------
-// Launch shape of the Navier-Stokes kernels.  zs = 2 splits each (element,
-// x, y) column between two threads (z-levels and flux points by halves),
-// doubling the warps per CTA for the same shared memory; minb is the CTAs per
-// SM the register allocation is held to (0: the compiler's choice).  Chosen by
-// timing P3 on B200: the split pays for the gradient kernel in both
-// precisions and for the face kernel in FP64 only.  The FP64 face kernel is
-// held to three CTAs per SM (80 registers; some of the RK update's values
-// spill): 0.43 against 0.47 ms per residual at two CTAs, 0.57 at four.
+// Launch shape of the Navier-Stokes kernels.  zs threads share each (element,
+// x, y) column (z-levels and flux points dealt out between them), multiplying
+// the warps per CTA for the same shared memory; minb is the CTAs per SM the
+// register allocation is held to (0: the compiler's choice).  Timed on B200,
+// us per residual on jittered boxes (P2 29^3, P4 20^3), zs = 1 -> this table:
+//   gradient  P2 FP64 219 -> 145, mixed 115 -> 82; P4 FP64 227 -> 217 (LDG
+//             beta 0.3: 246 -> 220), mixed 133 -> 118 (127 -> 109)
+//   face      P2 FP64 33 -> 33 (with the RK update 82 -> 57); mixed stays at
+//             one thread (20 against 25); P4 FP64 44 -> 41 (140 -> 90), mixed
+//             27 -> 25 (61 -> 50)
+// P1 and P3 split their columns in two: in both precisions for the gradient
+// kernel, in FP64 only for the face kernel, which is held to three CTAs per
+// SM (80 registers; some of the RK update's values spill): P3 64^3 0.43
+// against 0.47 ms per residual at two CTAs, 0.57 at four.  P4 with three
+// threads per column spills (96 registers): 262.
 // ---------------------------------------------------------------------------
 template <typename A, int N>
 struct HexNsShape
 {
-  static constexpr int grad_zs = (N % 2 == 0) ? 2 : 1;
-  static constexpr int grad_minb = grad_zs == 2 ? (sizeof(A) == 4 ? 4 : 2) : 0;
-  static constexpr int face_zs = (N % 2 == 0 && sizeof(A) == 8) ? 2 : 1;
-  static constexpr int face_minb = face_zs == 2 ? 3 : 0;
+  static constexpr bool f64 = sizeof(A) == 8;
+  static constexpr int grad_zs = N == 3 ? 3 : 2;
+  static constexpr int grad_minb = N == 3 ? (f64 ? 2 : 4) : N == 5 ? (f64 ? 1 : 2) : (f64 ? 2 : 4);
+  static constexpr int face_zs = f64 ? (N == 3 ? 3 : 2) : (N == 5 ? 2 : 1);
+  static constexpr int face_minb = f64 ? (N == 3 ? 4 : N == 5 ? 2 : 3) : (N == 5 ? 2 : 0);
 };
 
 // ---------------------------------------------------------------------------
@@ -573,7 +617,8 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
 {
   using H = HexIdx<N>;
   constexpr int ZS = HexNsShape<A, N>::grad_zs;
-  constexpr int S = H::S, Fp = H::Fp, V = 5, NZ = N / ZS;
+  using Z = ZSplit<N, ZS>;
+  constexpr int S = H::S, Fp = H::Fp, V = 5, NZ = Z::NZ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sU = reinterpret_cast<A *>(smem_raw);   // [S][V][TW]
   A *sUC = sU + S * V * TW;                  // [Fp][V][TW] common solution
@@ -583,7 +628,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
   // which would otherwise fall in one bank group
   const auto xo = [](int p) { return p * V * TW + TW * (p / H::N2); };
   const int l = threadIdx.x % TW, c = (threadIdx.x / TW) % H::N2, zs = threadIdx.x / (TW * H::N2);
-  const int ix = c % N, iy = c / N, iz0 = zs * NZ;
+  const int ix = c % N, iy = c / N, iz0 = zs * NZ, iz1 = Z::even ? iz0 + NZ : min(N, iz0 + NZ);
   const int64_t tile = blockIdx.x;
   if (tile >= a.ntiles) return;
   // the tile's metrics (gradient and flux passes) and face geometry (viscous
@@ -610,12 +655,13 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
     const T *Ut = a.U + tile * (int64_t)S * V * TW;
 #pragma unroll
     for (int k = 0; k < NZ; k++)
+      if (Z::even || iz0 + k < N)
 #pragma unroll
-      for (int v = 0; v < V; v++)
-      {
-        const int s = ix + N * iy + H::N2 * (iz0 + k);
-        sU[(s * V + v) * TW + l] = Ut[(s * V + v) * TW + l];
-      }
+        for (int v = 0; v < V; v++)
+        {
+          const int s = ix + N * iy + H::N2 * (iz0 + k);
+          sU[(s * V + v) * TW + l] = Ut[(s * V + v) * TW + l];
+        }
   }
   // common solution at own flux points (LDG, flip_beta = 1).  The points'
   // connectivity codes stay in registers for the viscous pass.
@@ -734,7 +780,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
   // corrected reference gradient -> physical gradient
   const int fzm = H::fpt(0, ix, iy), fzp = H::fpt(1, ix, iy);
 #pragma unroll 1
-  for (int iz = iz0; iz < iz0 + NZ; iz++)
+  for (int iz = iz0; iz < iz1; iz++)
   {
     const int s = ix + N * iy + H::N2 * iz;
     const int fxm = H::fxm(iy, iz), fxp = H::fxp(iy, iz), fym = H::fym(ix, iz), fyp = H::fyp(ix, iz);
@@ -911,7 +957,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
   __syncthreads();
   // flux at own column, transformed F~ = adj F (overwrites the gradient in place)
 #pragma unroll 1
-  for (int iz = iz0; iz < iz0 + NZ; iz++)
+  for (int iz = iz0; iz < iz1; iz++)
   {
     const int s = ix + N * iy + H::N2 * iz;
     A dU[V][3], F[V][3], P, Pp, Us[V], Ua[V], adj[3][3], det;
@@ -940,7 +986,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
   __syncthreads();
   // volume divergence
 #pragma unroll 1
-  for (int iz = iz0; iz < iz0 + NZ; iz++)
+  for (int iz = iz0; iz < iz1; iz++)
   {
     const int s = ix + N * iy + H::N2 * iz;
     A *out = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
@@ -989,7 +1035,8 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsS
 {
   using H = HexIdx<N>;
   constexpr int ZS = HexNsShape<A, N>::face_zs;
-  constexpr int S = H::S, Fp = H::Fp, V = 5, NZ = N / ZS;
+  using Z = ZSplit<N, ZS>;
+  constexpr int S = H::S, Fp = H::Fp, V = 5, NZ = Z::NZ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sFc = reinterpret_cast<A *>(smem_raw);  // [Fp][V][TW]
   A *sUnew = sFc + Fp * V * TW;              // [S][V][TW]
@@ -1012,6 +1059,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsS
 #pragma unroll
   for (int k = 0; k < NZ; k++)
   {
+    if (!Z::even && zs * NZ + k >= N) continue;
     const int s = ix + N * iy + H::N2 * (zs * NZ + k);
     const A *dv = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
 #pragma unroll
@@ -1021,6 +1069,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsS
   for (int k = 0; k < NZ; k++)
   {
     const int iz = zs * NZ + k;
+    if (!Z::even && iz >= N) continue;
     const int s = ix + N * iy + H::N2 * iz;
     A res[V];
 #pragma unroll

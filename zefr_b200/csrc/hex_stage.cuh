@@ -1,0 +1,87 @@
+// Launches of the hexahedral residual kernels of one arithmetic type.
+#pragma once
+#include "ctx_impl.cuh"
+#include "hex_kernels.cuh"
+#include "time_kernels.cuh"
+
+namespace zb {
+
+template <typename T, typename A, int N>
+static void launch_extrap_hex(Ctx &c)
+{
+  ProfScope ps(c, ZB_K_EXTRAP);
+  dev::k_hex_extrap<T, A, N><<<(unsigned)c.ntiles, TW * N * N, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur],
+                                                                              c.ntiles, line_ops<A, N>(c.plan));
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
+template <typename T, typename A, int N>
+static void launch_stage_hex(Ctx &c, const StageCfg &sc)
+{
+  using G = Shape<3, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V;
+  const Args<T, A> a = make_args<T, A>(c, sc);
+  const LineOpsT<A, N> ops = line_ops<A, N>(c.plan);
+  // hexahedra: column-mapped kernels, TW x N^2 threads per tile
+  constexpr int HT = TW * N * N;
+  if (!c.plan.params.viscous)
+  {
+    const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(A);
+    set_smem(dev::k_hex_euler<T, A, N>, smem);
+    ProfScope ps(c, ZB_K_EULER);
+    dev::k_hex_euler<T, A, N><<<(unsigned)c.ntiles, HT * dev::HexEulerShape<A, N>::zs, smem, c.stream>>>(a, ops);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  else
+  {
+    constexpr int ZG = dev::HexNsShape<A, N>::grad_zs, ZF = dev::HexNsShape<A, N>::face_zs;
+    const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(A);  // + sX padding
+    set_smem(dev::k_hex_ns_grad<T, A, N>, smem1);
+    if (!sc.face_only)
+    {
+      ProfScope ps(c, ZB_K_NS_GRAD);
+      dev::k_hex_ns_grad<T, A, N><<<(unsigned)c.ntiles, HT * ZG, smem1, c.stream>>>(a, ops);
+      c.launches++;
+      CK(cudaGetLastError());
+    }
+    if (sc.grad_only) return;
+    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A);
+    set_smem(dev::k_hex_ns_face<T, A, N>, smem2);
+    ProfScope ps(c, ZB_K_NS_FACE);
+    dev::k_hex_ns_face<T, A, N><<<(unsigned)c.ntiles, HT * ZF, smem2, c.stream>>>(a, ops);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  if (sc.extrap_next)
+  {
+    if (a.Fcom)
+      c.ufp_valid = false;  // the state changed and no traces were stored
+    else
+      c.cur ^= 1;
+  }
+}
+
+template <typename T, typename A, int N>
+static void bind_hex_order(Ctx &c)
+{
+  c.launch_extrap = &launch_extrap_hex<T, A, N>;
+  c.launch_stage = &launch_stage_hex<T, A, N>;
+  c.launch_dt = &launch_dt_impl<T, A, 3, N>;
+}
+
+template <typename T, typename A>
+static void bind_hex(Ctx &c)
+{
+  switch (c.N)
+  {
+    case 2: bind_hex_order<T, A, 2>(c); break;
+    case 3: bind_hex_order<T, A, 3>(c); break;
+    case 4: bind_hex_order<T, A, 4>(c); break;
+    case 5: bind_hex_order<T, A, 5>(c); break;
+    default: break;
+  }
+}
+
+}  // namespace zb

@@ -240,7 +240,7 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
       const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(double);
       NA_CK(cudaFuncSetAttribute(dev::k_hex_euler<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-      dev::k_hex_euler<double, double, N><<<(unsigned)p.ntiles, HT, smem, st>>>(a, ops);
+      dev::k_hex_euler<double, double, N><<<(unsigned)p.ntiles, HT * dev::HexEulerShape<double, N>::zs, smem, st>>>(a, ops);
       NA_CK(cudaGetLastError());
     }
     else

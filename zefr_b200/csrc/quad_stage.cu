@@ -1,0 +1,88 @@
+// Launches of the quadrilateral residual kernels.
+#include "ctx_impl.cuh"
+#include "time_kernels.cuh"
+
+namespace zb {
+
+template <typename T, typename A, int N>
+static void launch_extrap_quad(Ctx &c)
+{
+  const int64_t work = c.ntiles * Shape<2, N>::Fp * TW;
+  ProfScope ps(c, ZB_K_EXTRAP);
+  dev::k_extrap<T, A, 2, N><<<grid_for(work, 256), 256, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles,
+                                                                       line_ops<A, N>(c.plan));
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
+template <typename T, typename A, int N>
+static void launch_stage_quad(Ctx &c, const StageCfg &sc)
+{
+  constexpr int D = 2;
+  using G = Shape<D, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V, NT = G::NT;
+  const Args<T, A> a = make_args<T, A>(c, sc);
+  const LineOpsT<A, N> ops = line_ops<A, N>(c.plan);
+  const size_t ops_bytes = sizeof(LineOpsT<A, N>);
+  if (!c.plan.params.viscous)
+  {
+    const size_t smem = (size_t)(S * V + D * S * V + Fp * V) * TW * sizeof(A) + ops_bytes;
+    set_smem(dev::k_euler<T, A, D, N>, smem);
+    ProfScope ps(c, ZB_K_EULER);
+    dev::k_euler<T, A, D, N><<<(unsigned)c.ntiles, NT, smem, c.stream>>>(a, ops);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  else
+  {
+    const size_t smem1 = (size_t)(S * V + Fp * V + D * S * V) * TW * sizeof(A) + ops_bytes;
+    set_smem(dev::k_ns_grad<T, A, D, N>, smem1);
+    if (!sc.face_only)
+    {
+      ProfScope ps(c, ZB_K_NS_GRAD);
+      dev::k_ns_grad<T, A, D, N><<<(unsigned)c.ntiles, NT, smem1, c.stream>>>(a, ops);
+      c.launches++;
+      CK(cudaGetLastError());
+    }
+    if (sc.grad_only) return;
+    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A) + ops_bytes;
+    set_smem(dev::k_ns_face<T, A, D, N>, smem2);
+    ProfScope ps(c, ZB_K_NS_FACE);
+    dev::k_ns_face<T, A, D, N><<<(unsigned)c.ntiles, NT, smem2, c.stream>>>(a, ops);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  if (sc.extrap_next) c.cur ^= 1;
+}
+
+template <typename T, typename A, int N>
+static void bind_quad_order(Ctx &c)
+{
+  c.launch_extrap = &launch_extrap_quad<T, A, N>;
+  c.launch_stage = &launch_stage_quad<T, A, N>;
+  c.launch_dt = &launch_dt_impl<T, A, 2, N>;
+}
+
+template <typename T, typename A>
+static void bind_quad_t(Ctx &c)
+{
+  switch (c.N)
+  {
+    case 2: bind_quad_order<T, A, 2>(c); break;
+    case 3: bind_quad_order<T, A, 3>(c); break;
+    case 4: bind_quad_order<T, A, 4>(c); break;
+    case 5: bind_quad_order<T, A, 5>(c); break;
+    case 6: bind_quad_order<T, A, 6>(c); break;
+    default: break;
+  }
+}
+
+void bind_quad(Ctx &c)
+{
+  if (c.prec == ZB_FP64)
+    bind_quad_t<double, double>(c);
+  else
+    bind_quad_t<float, float>(c);
+}
+
+}  // namespace zb

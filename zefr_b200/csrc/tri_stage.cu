@@ -1,0 +1,103 @@
+// Launches of the triangle residual kernels.
+#include "ctx_impl.cuh"
+#include "tri_kernels.cuh"
+#include "tri_tc_kernels.cuh"
+
+namespace zb {
+
+// Triangles: dense-operator kernels (tri_kernels.cuh)
+template <typename T, typename A, int N>
+static void launch_extrap_tri(Ctx &c)
+{
+  using G = dev::TriShape<N>;
+  ProfScope ps(c, ZB_K_EXTRAP);
+  dev::k_tri_extrap<T, A, N><<<grid_for(c.ntiles * G::Fp * TW, 128), 128, 0, c.stream>>>(
+      (const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles, (const A *)c.dops);
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
+template <typename T, typename A, int N>
+static void launch_stage_tri(Ctx &c, const StageCfg &sc)
+{
+  using G = dev::TriShape<N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2;
+  const Args<T, A> a = make_args<T, A>(c, sc);
+  if (c.tc_err_host && *c.tc_err_host)
+  {
+    *c.tc_err_host = 0;
+    ZB_THROW(ZB_ERR_CUDA, "a tensor-core completion wait of an earlier launch timed out");
+  }
+  const size_t ops = (size_t)G::OPS_PAD;
+  if (!c.plan.params.viscous)
+  {
+    const size_t smem = (ops + (size_t)(S * V + D * S * V + Fp * V) * TW) * sizeof(A);
+    set_smem(dev::k_tri_euler<T, A, N>, smem);
+    ProfScope ps(c, ZB_K_EULER);
+    dev::k_tri_euler<T, A, N><<<(unsigned)c.ntiles, 128, smem, c.stream>>>(a);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  else
+  {
+    const size_t smem1 = (ops + (size_t)(S * V + Fp * V + D * S * V) * TW) * sizeof(A);
+    if (!sc.face_only)
+    {
+      ProfScope ps(c, ZB_K_NS_GRAD);
+      bool launched = false;
+      if constexpr (std::is_same<A, float>::value && N <= 5)
+      {
+        if (c.plan.params.tensor_ops)
+        {
+          using C = dev::TriTc<N>;
+          set_smem(dev::k_tri_ns_grad_tc<N>, C::SMEM);
+          const int64_t groups = (c.ntiles + C::TILES - 1) / C::TILES;
+          dev::k_tri_ns_grad_tc<N><<<(unsigned)groups, C::NT, C::SMEM, c.stream>>>(a);
+          launched = true;
+        }
+      }
+      if (!launched)
+      {
+        set_smem(dev::k_tri_ns_grad<T, A, N>, smem1);
+        dev::k_tri_ns_grad<T, A, N><<<(unsigned)c.ntiles, 128, smem1, c.stream>>>(a);
+      }
+      c.launches++;
+      CK(cudaGetLastError());
+    }
+    if (sc.grad_only) return;
+    const size_t smem2 = (ops + (size_t)(Fp * V + S * V) * TW) * sizeof(A);
+    set_smem(dev::k_tri_ns_face<T, A, N>, smem2);
+    ProfScope ps(c, ZB_K_NS_FACE);
+    dev::k_tri_ns_face<T, A, N><<<(unsigned)c.ntiles, 128, smem2, c.stream>>>(a);
+    c.launches++;
+    CK(cudaGetLastError());
+  }
+  if (sc.extrap_next) c.cur ^= 1;
+}
+
+template <typename T, typename A>
+static void bind_tri_t(Ctx &c)
+{
+#define ZB_BIND_TRI(NN)                             \
+  case NN:                                          \
+    c.launch_extrap = &launch_extrap_tri<T, A, NN>; \
+    c.launch_stage = &launch_stage_tri<T, A, NN>;   \
+    break;
+  switch (c.N)
+  {
+    ZB_BIND_TRI(2) ZB_BIND_TRI(3) ZB_BIND_TRI(4) ZB_BIND_TRI(5) ZB_BIND_TRI(6) ZB_BIND_TRI(7) ZB_BIND_TRI(8)
+    ZB_BIND_TRI(9)
+    default: break;
+  }
+#undef ZB_BIND_TRI
+}
+
+void bind_tri(Ctx &c)
+{
+  if (c.prec == ZB_FP64)
+    bind_tri_t<double, double>(c);
+  else
+    bind_tri_t<float, float>(c);
+}
+
+}  // namespace zb
