@@ -532,60 +532,135 @@ ZB_HD void visc_normal_vjp(const double U[D + 2], const double dU[D + 2][D], con
   flux_visc_vjp<D>(U, dU, Fb, ph, Ub, dUb);
 }
 
+// Free-stream parameters a boundary state depends on: k = 0 rho_fs,
+// 1..3 V_fs[k-1], 4 P_fs.  Only far-field (3) and characteristic (2) faces.
+ZB_HD bool bc_uses_freestream(int bc) { return bc == 2 || bc == 3; }
+
+ZB_HD void seed_param(Phys<Dual<double>> &q, int k)
+{
+  if (k == 0)
+    q.rho_fs.d = 1.0;
+  else if (k <= 3)
+    q.V_fs[k - 1].d = 1.0;
+  else
+    q.P_fs.d = 1.0;
+}
+
+// Reverse of ghost_grad: dUb += (d dUB / d dU)^T gB, Ub += (d dUB / d U)^T gB.
+template <int D>
+ZB_HD void ghost_grad_vjp(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
+                          const double gB[D + 2][D], double Ub[D + 2], double dUb[D + 2][D])
+{
+  for (int v = 0; v < D + 2; v++)
+    for (int d = 0; d < D; d++) dUb[v][d] += gB[v][d];
+  if (bc != 7 && bc != 9) return;
+  // dUB_E = dU_E - (dT . n) n with dT_j = dU_E,j - sum_i u_i dU_i,j + dU_0,j (|u|^2 - E / rho)
+  const double ir = 1.0 / U[0], e = U[D + 1] * ir;
+  double vel[D], velb[D], q2 = 0.0, dTnb = 0.0, eb = 0.0;
+  for (int d = 0; d < D; d++)
+  {
+    vel[d] = U[d + 1] * ir;
+    velb[d] = 0.0;
+    q2 += vel[d] * vel[d];
+    dTnb -= gB[D + 1][d] * n[d];
+  }
+  for (int j = 0; j < D; j++)
+  {
+    const double b = dTnb * n[j];
+    dUb[D + 1][j] += b;
+    dUb[0][j] += b * (q2 - e);
+    eb -= b * dU[0][j];
+    for (int i = 0; i < D; i++)
+    {
+      dUb[i + 1][j] -= b * vel[i];
+      velb[i] += b * (2.0 * dU[0][j] * vel[i] - dU[i + 1][j]);
+    }
+  }
+  Ub[D + 1] += eb * ir;
+  Ub[0] -= eb * e * ir;
+  for (int i = 0; i < D; i++)
+  {
+    Ub[i + 1] += velb[i] * ir;
+    Ub[0] -= velb[i] * vel[i] * ir;
+  }
+}
+
 // Boundary face, everything the own trace (U, dU) feeds:
-//   convective common flux with the ghost state, plus for viscous runs
+//   convective common flux with the ghost state UR, plus for viscous runs
 //   F_visc(UB, ghost_grad(U, dU)) . n + tau (U - UB).
+// The fluxes are reversed by hand (Riemann solver, viscous flux, boundary
+// gradient); only the ghost states, a map of the V state variables and the
+// free-stream parameters, go through dual numbers, one pass per input.  With
+// pb != nullptr also pb[k] += d (w . phi) / d param_k (seed_param's order).
+// A pass per input of the whole face function -- V (1 + D) and five more for
+// the parameters -- put 16 of them in series on a 2D viscous point and set the
+// time of every tile on a boundary (k_adj_ns1 on the 48 x 96 cylinder 223 us;
+// this form 74 us).
 template <int D, bool VISC>
 ZB_HD_INLINE void bnd_face_vjp_body(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                                    const double w[D + 2], const Phys<Dual<double>> &pd,
-                                    double Ub[D + 2], double dUb[D + 2][D])
+                                    const double w[D + 2], const Phys<double> &ph, double Ub[D + 2],
+                                    double dUb[D + 2][D], double *pb)
 {
   constexpr int V = D + 2;
   using DD = Dual<double>;
-  constexpr int NI = VISC ? V + V * D : V;
-  DD nd[D];
-  for (int d = 0; d < D; d++) nd[d] = DD(n[d]);
-  for (int k = 0; k < NI; k++)
+  double UR[V], UB[V], bR[V], bB[V];
+  ghost_state<double, D>(bc, U, n, UR, UB, ph);
+  for (int v = 0; v < V; v++) bR[v] = bB[v] = 0.0;
+  if (ph.fconv == 2)
+    roe_vjp<D>(U, UR, n, w, ph, Ub, bR);
+  else
+    rusanov_vjp<D>(U, UR, n, w, ph, Ub, bR);
+  if (VISC)
   {
-    DD L[V], dL[V][D], F[V];
+    double dUB[V][D], gB[V][D];
+    ghost_grad<double, D>(bc, U, dU, n, dUB);
+    for (int v = 0; v < V; v++)
+      for (int d = 0; d < D; d++) gB[v][d] = 0.0;
+    visc_normal_vjp<D>(UB, dUB, n, w, ph, bB, gB);
+    ghost_grad_vjp<D>(bc, U, dU, n, gB, Ub, dUb);
     for (int v = 0; v < V; v++)
     {
-      L[v] = DD(U[v], v == k ? 1.0 : 0.0);
-      for (int d = 0; d < D; d++) dL[v][d] = DD(dU[v][d], (k == V + v * D + d) ? 1.0 : 0.0);
+      Ub[v] += ph.ldg_tau * w[v];
+      bB[v] -= ph.ldg_tau * w[v];
     }
-    conv_face<D, DD>(bc, L, L, nd, F, pd);
-    if (VISC)
-    {
-      DD UR[V], UB[V], dUB[V][D], Fn[V];
-      ghost_state<DD, D>(bc, L, nd, UR, UB, pd);
-      ghost_grad<DD, D>(bc, L, dL, nd, dUB);
-      visc_normal<DD, D>(UB, dUB, nd, Fn, pd);
-      for (int v = 0; v < V; v++) F[v] += Fn[v] + pd.ldg_tau * (L[v] - UB[v]);
-    }
+  }
+  DD nd[D];
+  for (int d = 0; d < D; d++) nd[d] = DD(n[d]);
+  const int np = pb && bc_uses_freestream(bc) ? 5 : 0;
+#pragma unroll 1
+  for (int k = 0; k < V + np; k++)
+  {
+    const int kp = k - V;
+    if (kp >= 1 && kp <= 3 && kp > D) continue;
+    Phys<DD> q = dual_phys(ph);
+    if (kp >= 0) seed_param(q, kp);
+    DD L[V], R[V], B[V];
+    for (int v = 0; v < V; v++) L[v] = DD(U[v], v == k ? 1.0 : 0.0);
+    ghost_state<DD, D>(bc, L, nd, R, B, q);
     double acc = 0.0;
-    for (int v = 0; v < V; v++) acc += w[v] * F[v].d;
-    if (k < V)
-      Ub[k] += acc;
-    else
-      dUb[(k - V) / D][(k - V) % D] += acc;
+    for (int v = 0; v < V; v++) acc += bR[v] * R[v].d + (VISC ? bB[v] * B[v].d : 0.0);
+    // constant indices keep both arrays in registers
+    for (int v = 0; v < V; v++) Ub[v] += v == k ? acc : 0.0;
+    if (kp >= 0)
+      for (int j = 0; j < 5; j++) pb[j] += j == kp ? acc : 0.0;
   }
 }
 template <int D, bool VISC>
 ZB_HD_COLD void bnd_face_vjp_cold(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                                  const double w[D + 2], const Phys<Dual<double>> &pd,
-                                  double Ub[D + 2], double dUb[D + 2][D])
+                                  const double w[D + 2], const Phys<double> &ph, double Ub[D + 2],
+                                  double dUb[D + 2][D], double *pb)
 {
-  bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, pd, Ub, dUb);
+  bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
 }
 template <int D, bool VISC>
 ZB_HD_INLINE void bnd_face_vjp(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                               const double w[D + 2], const Phys<Dual<double>> &pd,
-                               double Ub[D + 2], double dUb[D + 2][D])
+                               const double w[D + 2], const Phys<double> &ph, double Ub[D + 2],
+                               double dUb[D + 2][D], double *pb)
 {
   if constexpr (D == 2)
-    bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, pd, Ub, dUb);
+    bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
   else
-    bnd_face_vjp_cold<D, VISC>(bc, U, dU, n, w, pd, Ub, dUb);
+    bnd_face_vjp_cold<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
 }
 
 // Ub += (d UB / d U)^T w for the prescribed boundary state UB of the LDG
@@ -622,72 +697,6 @@ ZB_HD_INLINE void bnd_ucomm_vjp(int bc, const double U[D + 2], const double n[D]
     bnd_ucomm_vjp_body<D>(bc, U, n, w, pd, Ub);
   else
     bnd_ucomm_vjp_cold<D>(bc, U, n, w, pd, Ub);
-}
-
-// Free-stream parameters a boundary state depends on: k = 0 rho_fs,
-// 1..3 V_fs[k-1], 4 P_fs.  Only far-field (3) and characteristic (2) faces.
-ZB_HD bool bc_uses_freestream(int bc) { return bc == 2 || bc == 3; }
-
-ZB_HD void seed_param(Phys<Dual<double>> &q, int k)
-{
-  if (k == 0)
-    q.rho_fs.d = 1.0;
-  else if (k <= 3)
-    q.V_fs[k - 1].d = 1.0;
-  else
-    q.P_fs.d = 1.0;
-}
-
-// pb[k] += d (w . phi) / d param_k for the boundary face function of
-// bnd_face_vjp.
-template <int D, bool VISC>
-ZB_HD_INLINE void bnd_face_param_vjp_body(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                                          const double w[D + 2], const Phys<Dual<double>> &pd, double pb[5])
-{
-  constexpr int V = D + 2;
-  using DD = Dual<double>;
-  if (!bc_uses_freestream(bc)) return;
-  DD nd[D], L[V], dL[V][D];
-  for (int d = 0; d < D; d++) nd[d] = DD(n[d]);
-  for (int v = 0; v < V; v++)
-  {
-    L[v] = DD(U[v]);
-    for (int d = 0; d < D; d++) dL[v][d] = DD(dU[v][d]);
-  }
-  for (int k = 0; k < 5; k++)
-  {
-    if (k >= 1 && k <= 3 && k > D) continue;
-    Phys<DD> q = pd;
-    seed_param(q, k);
-    DD F[V];
-    conv_face<D, DD>(bc, L, L, nd, F, q);
-    if (VISC)
-    {
-      DD UR[V], UB[V], dUB[V][D], Fn[V];
-      ghost_state<DD, D>(bc, L, nd, UR, UB, q);
-      ghost_grad<DD, D>(bc, L, dL, nd, dUB);
-      visc_normal<DD, D>(UB, dUB, nd, Fn, q);
-      for (int v = 0; v < V; v++) F[v] += Fn[v] + q.ldg_tau * (L[v] - UB[v]);
-    }
-    double acc = 0.0;
-    for (int v = 0; v < V; v++) acc += w[v] * F[v].d;
-    pb[k] += acc;
-  }
-}
-template <int D, bool VISC>
-ZB_HD_COLD void bnd_face_param_vjp_cold(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                                        const double w[D + 2], const Phys<Dual<double>> &pd, double pb[5])
-{
-  bnd_face_param_vjp_body<D, VISC>(bc, U, dU, n, w, pd, pb);
-}
-template <int D, bool VISC>
-ZB_HD_INLINE void bnd_face_param_vjp(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
-                                     const double w[D + 2], const Phys<Dual<double>> &pd, double pb[5])
-{
-  if constexpr (D == 2)
-    bnd_face_param_vjp_body<D, VISC>(bc, U, dU, n, w, pd, pb);
-  else
-    bnd_face_param_vjp_cold<D, VISC>(bc, U, dU, n, w, pd, pb);
 }
 
 // pb[k] += d (w . UB) / d param_k for the LDG boundary common solution.
@@ -1198,8 +1207,7 @@ __global__ void __launch_bounds__(Shape<D, N>::NT) k_adj_euler(const __grid_cons
       for (int v = 0; v < V; v++)
 #pragma unroll
         for (int d = 0; d < D; d++) dUz[v][d] = dUbz[v][d] = 0.0;
-      bnd_face_vjp<D, false>(-code - 1, Uo, dUz, n, w, dual_phys(a.ph), Ub, dUbz);
-      if (a.pbar) bnd_face_param_vjp<D, false>(-code - 1, Uo, dUz, n, w, dual_phys(a.ph), pb);
+      bnd_face_vjp<D, false>(-code - 1, Uo, dUz, n, w, a.ph, Ub, dUbz, a.pbar ? pb : nullptr);
     }
 #pragma unroll
     for (int v = 0; v < V; v++) sUbfp[(f * V + v) * TW + l] = Ub[v];
@@ -1497,8 +1505,7 @@ __global__ void __launch_bounds__(Shape<D, N>::NT) k_adj_ns1(const __grid_consta
     }
     else
     {
-      bnd_face_vjp<D, true>(-code - 1, Uo, dUo, n, w, dual_phys(a.ph), Ub, dUb);
-      if (a.pbar) bnd_face_param_vjp<D, true>(-code - 1, Uo, dUo, n, w, dual_phys(a.ph), pb);
+      bnd_face_vjp<D, true>(-code - 1, Uo, dUo, n, w, a.ph, Ub, dUb, a.pbar ? pb : nullptr);
     }
     if (GEO && a.gbar) geo_face_ns<D, N>(a, tile, f, l, code, n, w, Uo, dUo);
     double *ub = a.Ubfp + (tile * Fp + f) * (int64_t)V * TW + l;

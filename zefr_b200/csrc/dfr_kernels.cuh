@@ -689,8 +689,18 @@ __global__ void __launch_bounds__(Shape<D, N>::NT, (D == 3) ? 2 : 1) k_ns_grad(c
       visc_normal<A, D>(Ua, dUf, n, Fn, a.ph);
     else
     {
-      A UR[V], UB[V], dUB[V][D];
-      ghost_state<A, D>(-code - 1, Ua, n, UR, UB, a.ph);
+      A UB[V], dUB[V][D];
+      if constexpr (Pert<A>::on)
+      {
+        A UR[V];
+        ghost_state<A, D>(-code - 1, Ua, n, UR, UB, a.ph);
+      }
+      else
+      {
+        // the prescribed state is the point's common solution
+#pragma unroll
+        for (int v = 0; v < V; v++) UB[v] = sUC[(f * V + v) * TW + l];
+      }
       ghost_grad<A, D>(-code - 1, Ua, dUf, n, dUB);
       visc_normal<A, D>(UB, dUB, n, Fn, a.ph);
     }

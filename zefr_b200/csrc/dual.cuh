@@ -53,7 +53,7 @@ template <> ZB_HD Dual<double> dpow<Dual<double>>(Dual<double> x, Dual<double> y
 {
   // y is a constant exponent in every use (1.5, gamma, 1/(gamma-1))
   const double p = pow(x.v, y.v);
-  return {p, y.v * pow(x.v, y.v - 1.0) * x.d};
+  return {p, y.v * (x.v != 0.0 ? p / x.v : pow(x.v, y.v - 1.0)) * x.d};
 }
 
 template <typename T>

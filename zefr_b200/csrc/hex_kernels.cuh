@@ -912,8 +912,18 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
       visc_normal<A, 3>(Ua, dUf, n, Fn, a.ph);
     else
     {
-      A UR[V], UB[V], dUB[V][3];
-      ghost_state<A, 3>(-code - 1, Ua, n, UR, UB, a.ph);
+      A UB[V], dUB[V][3];
+      if constexpr (Pert<A>::on)
+      {
+        A UR[V];
+        ghost_state<A, 3>(-code - 1, Ua, n, UR, UB, a.ph);
+      }
+      else
+      {
+        // the prescribed state is the point's common solution
+#pragma unroll
+        for (int v = 0; v < V; v++) UB[v] = sUC[(fq * V + v) * TW + l];
+      }
       ghost_grad<A, 3>(-code - 1, Ua, dUf, n, dUB);
       visc_normal<A, 3>(UB, dUB, n, Fn, a.ph);
     }

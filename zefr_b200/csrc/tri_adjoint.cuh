@@ -172,8 +172,7 @@ __global__ void __launch_bounds__(128) k_tri_adj_euler(const __grid_constant__ A
       for (int v = 0; v < V; v++)
 #pragma unroll
         for (int d = 0; d < D; d++) dUz[v][d] = dUbz[v][d] = 0.0;
-      bnd_face_vjp<D, false>(-code - 1, Uo, dUz, n, w, dual_phys(a.ph), Ub, dUbz);
-      if (a.pbar) bnd_face_param_vjp<D, false>(-code - 1, Uo, dUz, n, w, dual_phys(a.ph), pb);
+      bnd_face_vjp<D, false>(-code - 1, Uo, dUz, n, w, a.ph, Ub, dUbz, a.pbar ? pb : nullptr);
     }
 #pragma unroll
     for (int v = 0; v < V; v++) sUbfp[(f * V + v) * TW + l] = Ub[v];
@@ -356,8 +355,7 @@ __global__ void __launch_bounds__(128) k_tri_adj_ns1(const __grid_constant__ Adj
     }
     else
     {
-      bnd_face_vjp<D, true>(-code - 1, Uo, dUo, n, w, dual_phys(a.ph), Ub, dUb);
-      if (a.pbar) bnd_face_param_vjp<D, true>(-code - 1, Uo, dUo, n, w, dual_phys(a.ph), pb);
+      bnd_face_vjp<D, true>(-code - 1, Uo, dUo, n, w, a.ph, Ub, dUb, a.pbar ? pb : nullptr);
     }
     double *ub = a.Ubfp + (tile * Fp + f) * (int64_t)V * TW + l;
     double *dub = a.dUbfp + (tile * Fp + f) * (int64_t)V * D * TW + l;

@@ -454,8 +454,14 @@ __global__ void __launch_bounds__(128) k_tri_ns_grad(const __grid_constant__ Arg
       visc_normal<A, D>(Ua, dUf, n, Fn, a.ph);
     else
     {
-      A UR[V], UB[V], dUB[V][D];
-      ghost_state<A, D>(-code - 1, Ua, n, UR, UB, a.ph);
+      A UB[V], dUB[V][D];
+      if constexpr (Pert<A>::on)
+      {
+        A UR[V];
+        ghost_state<A, D>(-code - 1, Ua, n, UR, UB, a.ph);
+      }
+      else
+        ld4(sUC + tvl<A>(f, l), UB);  // the prescribed state is the point's common solution
       ghost_grad<A, D>(-code - 1, Ua, dUf, n, dUB);
       visc_normal<A, D>(UB, dUB, n, Fn, a.ph);
     }
