@@ -230,6 +230,63 @@ ZB_HD void visc_normal(const T U[D + 2], const T dU[D + 2][D], const T n[D],
   }
 }
 
+// Inviscid flux through a face, F(U).n = [m.n, m u.n + p n, (E + p) u.n], of a
+// stored state, with the absolute pressure P, its deviation Pp, 1/rho and the
+// normal velocity un of the absolute state.  The perturbation form gives
+// F(U).n - F(Ur).n with the cancellation-free terms of flux_conv_pert taken
+// normal to the face first.  A third of the products of the full flux matrix
+// times n, and none of its D (D + 2) values held per side.
+template <typename T, int D>
+ZB_HD void flux_normal_stored(const T Us[D + 2], const T n[D], T Fn[D + 2], T &P, T &Pp, T &ir, T &un,
+                              const Phys<T> &ph)
+{
+  if constexpr (Pert<T>::on)
+  {
+    const T *Ur = ph.Ur;
+    ir = T(1) / (Ur[0] + Us[0]);
+    const T c = Us[0] * ir * ph.inv_rr;  // rho' / (rho rho_r)
+    T mrn = Ur[1] * n[0], mn = Us[1] * n[0], mrmp = Ur[1] * Us[1], mpmp = Us[1] * Us[1];
+#pragma unroll
+    for (int d = 1; d < D; d++)
+    {
+      mrn += Ur[d + 1] * n[d];
+      mn += Us[d + 1] * n[d];
+      mrmp += Ur[d + 1] * Us[d + 1];
+      mpmp += Us[d + 1] * Us[d + 1];
+    }
+    const T dke2 = (T(2) * mrmp + mpmp) * ir - ph.mr2 * c;
+    Pp = (ph.gamma - T(1)) * (Us[D + 1] - T(0.5) * dke2);
+    P = ph.Pr + Pp;
+    un = (mrn + mn) * ir;
+    const T ep = Us[D + 1] + Pp;
+    const T dun = mn * ir - mrn * c;  // u.n - u_r.n
+    Fn[0] = mn;
+#pragma unroll
+    for (int d = 0; d < D; d++) Fn[d + 1] = Ur[d + 1] * dun + Us[d + 1] * un + Pp * n[d];
+    Fn[D + 1] = ph.er * dun + ep * un;
+  }
+  else
+  {
+    T Ua[D + 2];
+    to_abs<T, D>(Us, Ua, ph);
+    ir = T(1) / Ua[0];
+    T mn = Ua[1] * n[0], m2 = Ua[1] * Ua[1];
+#pragma unroll
+    for (int d = 1; d < D; d++)
+    {
+      mn += Ua[d + 1] * n[d];
+      m2 += Ua[d + 1] * Ua[d + 1];
+    }
+    P = (ph.gamma - T(1)) * (Ua[D + 1] - T(0.5) * (m2 * ir));
+    Pp = P;
+    un = mn * ir;
+    Fn[0] = mn;
+#pragma unroll
+    for (int d = 0; d < D; d++) Fn[d + 1] = Ua[d + 1] * un + P * n[d];
+    Fn[D + 1] = (Ua[D + 1] + P) * un;
+  }
+}
+
 // Rusanov common normal flux, upwinded form (src/faces.cpp:1243-1364, rus_bias 0).
 // UL, UR are stored states (deviations from Ur in the perturbation form); the
 // result is the common flux of the stored form (minus F(Ur).n).
@@ -237,36 +294,15 @@ template <typename T, int D>
 ZB_HD void rusanov(const T UL[D + 2], const T UR[D + 2], const T n[D], T Fc[D + 2],
                                         const Phys<T> &ph)
 {
-  T FL[D + 2][D], FR[D + 2][D], PL, PR, QL, QR;
-  flux_conv_stored<T, D>(UL, FL, PL, QL, ph);
-  flux_conv_stored<T, D>(UR, FR, PR, QR, ph);
-  T AL[D + 2], AR[D + 2];
-  to_abs<T, D>(UL, AL, ph);
-  to_abs<T, D>(UR, AR, ph);
-  const T irL = T(1) / AL[0], irR = T(1) / AR[0];
+  T FL[D + 2], FR[D + 2], PL, PR, QL, QR, irL, irR, VnL, VnR;
+  flux_normal_stored<T, D>(UL, n, FL, PL, QL, irL, VnL, ph);
+  flux_normal_stored<T, D>(UR, n, FR, PR, QR, irR, VnR, ph);
   const T aL = dsqrt<T>(ph.gamma * PL * irL);
   const T aR = dsqrt<T>(ph.gamma * PR * irR);
-  T VnL = AL[1] * irL * n[0], VnR = AR[1] * irR * n[0];
-#pragma unroll
-  for (int d = 1; d < D; d++)
-  {
-    VnL += AL[d + 1] * irL * n[d];
-    VnR += AR[d + 1] * irR * n[d];
-  }
   const T eig = dmax<T>(dabs<T>(VnL) + aL, dabs<T>(VnR) + aR);
   const T diss = T(0.5) * eig * (T(1) - ph.rus_k);
 #pragma unroll
-  for (int v = 0; v < D + 2; v++)
-  {
-    T fl = FL[v][0] * n[0], fr = FR[v][0] * n[0];
-#pragma unroll
-    for (int d = 1; d < D; d++)
-    {
-      fl += FL[v][d] * n[d];
-      fr += FR[v][d] * n[d];
-    }
-    Fc[v] = T(0.5) * (fr + fl) - diss * (UR[v] - UL[v]);
-  }
+  for (int v = 0; v < D + 2; v++) Fc[v] = T(0.5) * (FR[v] + FL[v]) - diss * (UR[v] - UL[v]);
 }
 
 // Roe approximate Riemann solver (Roe 1981, J. Comput. Phys. 43:357) in the
@@ -287,9 +323,9 @@ ZB_HD void roe(const T SL[D + 2], const T SR[D + 2], const T n[D], T Fc[D + 2],
     return;
   }
   const T g = ph.gamma;
-  T FL[D + 2][D], FR[D + 2][D], PL, PR, QL, QR;
-  flux_conv_stored<T, D>(SL, FL, PL, QL, ph);
-  flux_conv_stored<T, D>(SR, FR, PR, QR, ph);
+  T FL[D + 2], FR[D + 2], PL, PR, QL, QR, irL, irR, unL, unR;
+  flux_normal_stored<T, D>(SL, n, FL, PL, QL, irL, unL, ph);
+  flux_normal_stored<T, D>(SR, n, FR, PR, QR, irR, unR, ph);
   T UL[D + 2], UR[D + 2];
   to_abs<T, D>(SL, UL, ph);
   to_abs<T, D>(SR, UR, ph);
@@ -297,17 +333,13 @@ ZB_HD void roe(const T SL[D + 2], const T SR[D + 2], const T n[D], T Fc[D + 2],
   const T sL = dsqrt<T>(rL), sR = dsqrt<T>(rR);
   const T inv = T(1) / (sL + sR);
   // one reciprocal per state: velocities and enthalpies by multiplication
-  const T irL = T(1) / rL, irR = T(1) / rR;
   T u[D], uL[D], uR[D];
-  T unL = T(0), unR = T(0);
 #pragma unroll
   for (int d = 0; d < D; d++)
   {
     uL[d] = UL[d + 1] * irL;
     uR[d] = UR[d + 1] * irR;
     u[d] = (sL * uL[d] + sR * uR[d]) * inv;
-    unL += uL[d] * n[d];
-    unR += uR[d] * n[d];
   }
   const T HL = (UL[D + 1] + PL) * irL, HR = (UR[D + 1] + PR) * irR;
   const T H = (sL * HL + sR * HR) * inv;
@@ -347,17 +379,7 @@ ZB_HD void roe(const T SL[D + 2], const T SR[D + 2], const T n[D], T Fc[D + 2],
   }
   diss[D + 1] = l1 * a1 * (H - a * un) + l2 * (a2w * T(0.5) * q2 + rho * udvt) + l3 * a3 * (H + a * un);
 #pragma unroll
-  for (int v = 0; v < D + 2; v++)
-  {
-    T fl = FL[v][0] * n[0], fr = FR[v][0] * n[0];
-#pragma unroll
-    for (int d = 1; d < D; d++)
-    {
-      fl += FL[v][d] * n[d];
-      fr += FR[v][d] * n[d];
-    }
-    Fc[v] = T(0.5) * (fl + fr) - T(0.5) * diss[v];
-  }
+  for (int v = 0; v < D + 2; v++) Fc[v] = T(0.5) * (FL[v] + FR[v]) - T(0.5) * diss[v];
 }
 
 // The same Roe flux in FP64 arithmetic on absolute states: the normal fluxes
