@@ -15,6 +15,7 @@
 #include <chrono>
 
 #include "ctx_impl.cuh"
+#include "quad_kernels.cuh"
 
 namespace zb {
 
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(256) k_batch_euler(const BatchCase<T, A> *__re
         have = w.x;
       }
       dev::group_sync(bar, gsz);
-      dev::euler_tile<T, A, 2, NN>(sbc->a, *reinterpret_cast<const LineOpsT<A, NN> *>(sbc->ops), w.y, tsm, tid, gsz,
+      dev::euler_tile<T, A, NN>(sbc->a, *reinterpret_cast<const LineOpsT<A, NN> *>(sbc->ops), w.y, tsm, tid, gsz,
                                    bar);
     }
   }
@@ -125,7 +126,7 @@ __global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 1) k_batch_euler_fus
       {
 #define ZB_TILE(NN)                                                                                              \
   case NN:                                                                                                       \
-    dev::euler_tile<T, A, 2, NN>(sbc->a, *reinterpret_cast<const LineOpsT<A, NN> *>(sbc->ops), w.y, tsm, tid, gsz, \
+    dev::euler_tile<T, A, NN>(sbc->a, *reinterpret_cast<const LineOpsT<A, NN> *>(sbc->ops), w.y, tsm, tid, gsz, \
                                  bar);                                                                           \
     break;
         ZB_TILE(2) ZB_TILE(3) ZB_TILE(4) ZB_TILE(5) ZB_TILE(6)
@@ -140,11 +141,11 @@ static size_t euler_smem_bytes(int N, size_t asz)
 {
   switch (N)
   {
-    case 2: return dev::euler_smem_elems<2, 2>() * asz;
-    case 3: return dev::euler_smem_elems<2, 3>() * asz;
-    case 4: return dev::euler_smem_elems<2, 4>() * asz;
-    case 5: return dev::euler_smem_elems<2, 5>() * asz;
-    default: return dev::euler_smem_elems<2, 6>() * asz;
+    case 2: return dev::euler_smem_elems<2>() * asz;
+    case 3: return dev::euler_smem_elems<3>() * asz;
+    case 4: return dev::euler_smem_elems<4>() * asz;
+    case 5: return dev::euler_smem_elems<5>() * asz;
+    default: return dev::euler_smem_elems<6>() * asz;
   }
 }
 

@@ -217,35 +217,62 @@ __device__ __forceinline__ void gather_fpt(const T *src, int pidx, A out[V])
   for (int v = 0; v < V; v++) out[v] = (A)src[(row + v) * TW + lane];
 }
 
-// ---------------------------------------------------------------------------
-// Extrapolate the state to flux points: U_fpts = oppE U_spts (src/elements.cpp:1337-1360)
-// ---------------------------------------------------------------------------
-template <typename T, typename A, int D, int N>
-__global__ void __launch_bounds__(256) k_extrap(const T *__restrict__ U, T *__restrict__ Ufp, int64_t ntiles,
-                                                const __grid_constant__ LineOpsT<A, N> ops)
+// Shared-memory tile arrays of the 2D kernels (states, common solutions,
+// gradients, fluxes) keep the variables of one (point, element) in 16-byte
+// groups, [P][4/W][TW][W] with W = 16 / sizeof(A): FP32 holds all four
+// variables in one group, FP64 two groups of two.  One 16-byte load per group
+// fetches a point's variables where the global [P][V][TW] order takes four
+// loads, and the eight elements of a warp's point read 128 contiguous bytes
+// per group (no bank conflicts).
+template <typename A>
+struct TVec
 {
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V;
-  const int64_t total = ntiles * Fp * TW;
-  for (int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += (int64_t)gridDim.x * blockDim.x)
-  {
-    const int l = (int)(gid % TW);
-    const int f = (int)((gid / TW) % Fp);
-    const int64_t tile = gid / ((int64_t)TW * Fp);
-    int dim, side, base, stride;
-    fpt_line<D, N>(f, dim, side, base, stride);
-    const T *Ut = U + tile * (int64_t)S * V * TW;
-    T *out = Ufp + (tile * Fp + f) * (int64_t)V * TW;
-#pragma unroll
-    for (int v = 0; v < V; v++)
-    {
-      A acc = (side < 0 ? ops.Em[0] : ops.Ep[0]) * (A)Ut[((base)*V + v) * TW + l];
-#pragma unroll
-      for (int m = 1; m < N; m++)
-        acc += (side < 0 ? ops.Em[m] : ops.Ep[m]) * (A)Ut[((base + m * stride) * V + v) * TW + l];
-      out[v * TW + l] = (T)acc;
-    }
-  }
+  static constexpr int W = 16 / (int)sizeof(A), G = 4 / W;
+};
+
+// offset of (point p, element l, variable v)
+template <typename A>
+__device__ __forceinline__ int tix(int p, int l, int v)
+{
+  return ((p * TVec<A>::G + v / TVec<A>::W) * TW + l) * TVec<A>::W + v % TVec<A>::W;
+}
+
+// offset of (point p, element l)'s first group
+template <typename A>
+__device__ __forceinline__ int tvl(int p, int l)
+{
+  return tix<A>(p, l, 0);
+}
+
+__device__ __forceinline__ void ld4(const float *p, float x[4])
+{
+  const float4 q = *reinterpret_cast<const float4 *>(p);
+  x[0] = q.x;
+  x[1] = q.y;
+  x[2] = q.z;
+  x[3] = q.w;
+}
+
+// the second group of two doubles sits TW groups further on
+__device__ __forceinline__ void ld4(const double *p, double x[4])
+{
+  const double2 a = *reinterpret_cast<const double2 *>(p);
+  const double2 b = *reinterpret_cast<const double2 *>(p + 2 * TW);
+  x[0] = a.x;
+  x[1] = a.y;
+  x[2] = b.x;
+  x[3] = b.y;
+}
+
+__device__ __forceinline__ void st4(float *p, const float x[4])
+{
+  *reinterpret_cast<float4 *>(p) = make_float4(x[0], x[1], x[2], x[3]);
+}
+
+__device__ __forceinline__ void st4(double *p, const double x[4])
+{
+  *reinterpret_cast<double2 *>(p) = make_double2(x[0], x[1]);
+  *reinterpret_cast<double2 *>(p + 2 * TW) = make_double2(x[2], x[3]);
 }
 
 // ---------------------------------------------------------------------------
@@ -295,13 +322,170 @@ __device__ __forceinline__ A step_dt(const Args<T, A> &a, int64_t tile, int l)
 }
 
 // ---------------------------------------------------------------------------
-// Store the residual of one point and apply the optional RK update
-// (src/solver.cpp:2916-2937, 3040-3094).
+// 2D faces (quadrilaterals and triangles: four variables, Fp flux points per
+// element)
 // ---------------------------------------------------------------------------
-template <typename T, typename A, int S, int V, int NM>
-__device__ __forceinline__ void store_rk(const Args<T, A> &a, int64_t tile, int s, int l, const A res[V], A *sUnew)
+
+// LDG common solution at own flux point f (flip_beta = 1) from the traces
+template <typename T, typename A>
+__device__ __forceinline__ void common_solution_2d(const Args<T, A> &a, int64_t tile, int Fp, int f, int l, int code,
+                                                   const A Uo[4], A UC[4])
 {
-  constexpr int D = NM == 5 ? 2 : 3, MAXPREV = 3;
+  const A beta = a.ph.ldg_b;
+  if (code >= 0)
+  {
+    const int slot = code & 1;
+    if ((beta == A(0.5) && slot) || (beta == A(-0.5) && !slot))
+    {
+      // beta = +1/2 (-1/2) takes the right (left) trace: the own one, no gather
+#pragma unroll
+      for (int v = 0; v < 4; v++) UC[v] = Uo[v];
+      return;
+    }
+    A Un[4];
+    gather_fpt<T, A, 4>(a.Ufp, code >> 1, Un);
+#pragma unroll
+    for (int v = 0; v < 4; v++)
+    {
+      const A ul = slot ? Un[v] : Uo[v];
+      const A ur = slot ? Uo[v] : Un[v];
+      if (beta == A(0.5))
+        UC[v] = ur;
+      else if (beta == A(-0.5))
+        UC[v] = ul;
+      else
+        UC[v] = A(0.5) * (ul + ur) - beta * (ul - ur);
+    }
+    return;
+  }
+  A n[2], Ua[4], URa[4], UBa[4];
+  const T *g = a.fgeo + (tile * Fp + f) * (int64_t)3 * TW + l;
+  n[0] = g[0];
+  n[1] = g[TW];
+  to_abs<A, 2>(Uo, Ua, a.ph);
+  ghost_state<A, 2>(-code - 1, Ua, n, URa, UBa, a.ph);
+  to_stored<A, 2>(UBa, UC, a.ph);
+}
+
+// whether this side forms the viscous normal flux of a point: not where
+// one-sided LDG takes the partner's
+template <typename A>
+__device__ __forceinline__ bool own_visc_flux(A beta, int code)
+{
+  return !(code >= 0 && ((beta == A(0.5) && (code & 1)) || (beta == A(-0.5) && !(code & 1))));
+}
+
+// viscous normal flux at own flux point f from its trace and gradient trace
+// (boundaries: of the prescribed state UC and gradient)
+template <typename T, typename A>
+__device__ __forceinline__ void visc_face_2d(const Args<T, A> &a, int64_t tile, int Fp, int f, int l, int code,
+                                             const A Uf[4], const A dUf[4][2], const A UC[4])
+{
+  A n[2], Ua[4], Fn[4];
+  const T *g = a.fgeo + (tile * Fp + f) * (int64_t)3 * TW + l;
+  n[0] = g[0];
+  n[1] = g[TW];
+  to_abs<A, 2>(Uf, Ua, a.ph);
+  if (code >= 0)
+    visc_normal<A, 2>(Ua, dUf, n, Fn, a.ph);
+  else
+  {
+    A UB[4], dUB[4][2];
+    if constexpr (Pert<A>::on)
+    {
+      A UR[4];
+      ghost_state<A, 2>(-code - 1, Ua, n, UR, UB, a.ph);
+    }
+    else
+    {
+      // the prescribed state is the point's common solution
+#pragma unroll
+      for (int v = 0; v < 4; v++) UB[v] = UC[v];
+    }
+    ghost_grad<A, 2>(-code - 1, Ua, dUf, n, dUB);
+    visc_normal<A, 2>(UB, dUB, n, Fn, a.ph);
+  }
+  T *out = a.Fvn + (tile * Fp + f) * (int64_t)4 * TW + l;
+#pragma unroll
+  for (int v = 0; v < 4; v++) out[v * TW] = Fn[v];
+}
+
+// convective (VISC: + LDG viscous) common flux at own flux point f, dA-scaled
+// and signed for this element
+template <typename T, typename A, bool VISC>
+__device__ __forceinline__ void common_flux_2d(const Args<T, A> &a, int64_t tile, int Fp, int f, int l, A out[4])
+{
+  constexpr int V = 4;
+  const int code = a.nbr[(tile * Fp + f) * (int64_t)TW + l];
+  const T *g = a.fgeo + (tile * Fp + f) * (int64_t)3 * TW + l;
+  const A n[2] = {g[0], g[TW]};
+  const A dA = g[2 * TW];
+  A Uo[V], Un[V], UL[V], UR[V], UB[V], Fc[V];
+  const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
+#pragma unroll
+  for (int v = 0; v < V; v++) Uo[v] = uo[v * TW];
+  if (code >= 0) gather_fpt<T, A, V>(a.Ufp, code >> 1, Un);
+  A F1[V], F2[V];
+  const A beta = a.ph.ldg_b, tau = a.ph.ldg_tau;
+  if (VISC)
+  {
+    // the viscous normal flux of the side(s) LDG takes, loaded with the traces
+    const bool own = own_visc_flux(beta, code);
+    const T *fvo = a.Fvn + (tile * Fp + f) * (int64_t)V * TW + l;
+#pragma unroll
+    for (int v = 0; v < V; v++) F1[v] = F2[v] = A(0);
+    if (own)
+    {
+#pragma unroll
+      for (int v = 0; v < V; v++) F1[v] = fvo[v * TW];
+    }
+    if (code >= 0 && (!own || (beta != A(0.5) && beta != A(-0.5)))) gather_fpt<T, A, V>(a.Fvn, code >> 1, F2);
+  }
+  conv_common<T, A, 2>(a, Uo, Un, code, n, UL, UR, UB, Fc);
+  const bool right = (code >= 0) && (code & 1);
+  if (VISC)
+  {
+#pragma unroll
+    for (int v = 0; v < V; v++)
+    {
+      const A FnL = right ? F2[v] : F1[v], FnR = right ? F1[v] : F2[v];
+      if (code >= 0)
+        Fc[v] += A(0.5) * (FnL + FnR) + tau * (UL[v] - UR[v]) + beta * (FnL - FnR);
+      else
+        Fc[v] += FnL + tau * (UL[v] - UB[v]);
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < V; v++) out[v] = right ? -Fc[v] * dA : Fc[v] * dA;
+}
+
+// ---------------------------------------------------------------------------
+// Store the residual of one point and apply the optional RK update
+// (src/solver.cpp:2916-2937, 3040-3094).  rk_load fetches what the update
+// needs besides the residual, ahead of the barrier before the surface terms.
+// ---------------------------------------------------------------------------
+template <typename A, int V>
+struct RkIn
+{
+  A detJ, u_ini[V];
+};
+
+template <typename T, typename A, int S, int V, int NM>
+__device__ __forceinline__ void rk_load(const Args<T, A> &a, int64_t tile, int s, int l, RkIn<A, V> &in)
+{
+  constexpr int D = NM == 5 ? 2 : 3;
+  const int64_t base = (tile * S + s) * (int64_t)V * TW;
+  in.detJ = a.mets[((tile * S + s) * NM + D * D) * TW + l];
+#pragma unroll
+  for (int v = 0; v < V; v++) in.u_ini[v] = a.save_ini ? (A)a.U[base + v * TW + l] : (A)a.U_ini[base + v * TW + l];
+}
+
+// unew: the updated state as stored
+template <typename T, typename A, int S, int V>
+__device__ __forceinline__ void store_rk(const Args<T, A> &a, int64_t tile, int s, int l, const A res[V],
+                                         const RkIn<A, V> &in, A unew[V])
+{
+  constexpr int MAXPREV = 3;
   const int64_t base = (tile * S + s) * (int64_t)V * TW;
   if (a.rk_mode == 0)
   {
@@ -311,17 +495,11 @@ __device__ __forceinline__ void store_rk(const Args<T, A> &a, int64_t tile, int 
   }
   // every load of the point before the first store: a load cannot move above
   // a store that may alias it, so interleaving them serialises the accesses
-  const A detJ = a.mets[((tile * S + s) * NM + D * D) * TW + l];
   const A dtv = step_dt(a, tile, l);
   const bool fast = a.rk_mode == 1 || a.nprev <= MAXPREV;
-  A u_ini[V], prev[MAXPREV][V], comp[V];
+  A prev[MAXPREV][V], comp[V];
 #pragma unroll
-  for (int v = 0; v < V; v++)
-  {
-    const int64_t idx = base + v * TW + l;
-    u_ini[v] = a.save_ini ? (A)a.U[idx] : (A)a.U_ini[idx];
-    comp[v] = (a.rk_mode == 2 && a.Ucomp) ? (A)a.Ucomp[idx] : A(0);
-  }
+  for (int v = 0; v < V; v++) comp[v] = (a.rk_mode == 2 && a.Ucomp) ? (A)a.Ucomp[base + v * TW + l] : A(0);
   if (a.rk_mode == 2 && fast)
   {
 #pragma unroll
@@ -334,14 +512,15 @@ __device__ __forceinline__ void store_rk(const Args<T, A> &a, int64_t tile, int 
   }
 #pragma unroll
   for (int v = 0; v < V; v++) a.divF[base + v * TW + l] = res[v];
+  const A c = dtv / in.detJ;
 #pragma unroll
   for (int v = 0; v < V; v++)
   {
     const int64_t idx = base + v * TW + l;
-    if (a.save_ini) a.U_ini[idx] = u_ini[v];
-    A unew;
+    if (a.save_ini) a.U_ini[idx] = in.u_ini[v];
+    A u;
     if (a.rk_mode == 1)
-      unew = u_ini[v] - a.rk_coef[0] * dtv / detJ * res[v];
+      u = in.u_ini[v] - a.rk_coef[0] * c * res[v];
     else if (a.Ucomp)
     {
       // Kahan-compensated accumulation of the step increment; the
@@ -351,540 +530,31 @@ __device__ __forceinline__ void store_rk(const Args<T, A> &a, int64_t tile, int 
       {
 #pragma unroll
         for (int st = 0; st < MAXPREV; st++)
-          if (st < a.nprev) delta -= a.rk_coef[st] * dtv / detJ * prev[st][v];
+          if (st < a.nprev) delta -= a.rk_coef[st] * c * prev[st][v];
       }
       else
-        for (int st = 0; st < a.nprev; st++) delta -= a.rk_coef[st] * dtv / detJ * (A)a.divF_prev[st][idx];
-      delta -= a.rk_coef[a.nprev] * dtv / detJ * res[v];
+        for (int st = 0; st < a.nprev; st++) delta -= a.rk_coef[st] * c * (A)a.divF_prev[st][idx];
+      delta -= a.rk_coef[a.nprev] * c * res[v];
       const A y = delta - comp[v];
-      unew = (A)(T)(u_ini[v] + y);
-      a.Ucomp[idx] = (T)((unew - u_ini[v]) - y);
+      u = (A)(T)(in.u_ini[v] + y);
+      a.Ucomp[idx] = (T)((u - in.u_ini[v]) - y);
     }
     else
     {
       // reference order: U = U_ini; U -= b_s dt/|J| divF_s for s = 0..
-      unew = u_ini[v];
+      u = in.u_ini[v];
       if (fast)
       {
 #pragma unroll
         for (int st = 0; st < MAXPREV; st++)
-          if (st < a.nprev) unew -= a.rk_coef[st] * dtv / detJ * prev[st][v];
+          if (st < a.nprev) u -= a.rk_coef[st] * c * prev[st][v];
       }
       else
-        for (int st = 0; st < a.nprev; st++) unew -= a.rk_coef[st] * dtv / detJ * a.divF_prev[st][idx];
-      unew -= a.rk_coef[a.nprev] * dtv / detJ * res[v];
+        for (int st = 0; st < a.nprev; st++) u -= a.rk_coef[st] * c * a.divF_prev[st][idx];
+      u -= a.rk_coef[a.nprev] * c * res[v];
     }
-    a.Uout[idx] = unew;
-    if (sUnew) sUnew[(s * V + v) * TW + l] = (A)(T)unew;  // the state as stored
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Final per-point residual: volume part + surface correction, then optional
-// RK update (src/solver.cpp:2916-2937, 3040-3094).
-// ---------------------------------------------------------------------------
-template <typename T, typename A, int D, int N>
-__device__ __forceinline__ void finish_point(const Args<T, A> &a, int64_t tile, int s, int l, const A vol[D + 2],
-                                             const A *sFc, const SOps<A, N> &o, A *sUnew)
-{
-  using G = Shape<D, N>;
-  constexpr int S = G::S, V = G::V, NM = G::NM;
-  A surf[V];
-#pragma unroll
-  for (int v = 0; v < V; v++) surf[v] = A(0);
-  // surface terms in ascending flux point order = ascending face order
-#pragma unroll
-  for (int face = 0; face < 2 * D; face++)
-  {
-    int dim, side;
-    face_dim_side<D>(face, dim, side);
-    int i, fm, fp;
-    spt_ends<D, N>(s, dim, i, fm, fp);
-    const int f = side < 0 ? fm : fp;
-    const A c = side < 0 ? -o.Dbm[i] : o.Dbp[i];
-#pragma unroll
-    for (int v = 0; v < V; v++) surf[v] += c * sFc[(f * V + v) * TW + l];
-  }
-  A res[V];
-#pragma unroll
-  for (int v = 0; v < V; v++) res[v] = vol[v] + surf[v];
-  store_rk<T, A, S, V, NM>(a, tile, s, l, res, sUnew);
-}
-
-template <typename T, typename A, int D, int N>
-__device__ __forceinline__ void extrap_next_tile(const Args<T, A> &a, int64_t tile, const A *sUnew, const SOps<A, N> &o,
-                                                 int tid, int nth)
-{
-  using G = Shape<D, N>;
-  constexpr int Fp = G::Fp, V = G::V;
-  for (int it = tid; it < Fp * TW; it += nth)
-  {
-    const int f = it / TW, l = it % TW;
-    T *out = a.Ufp_next + (tile * Fp + f) * (int64_t)V * TW;
-#pragma unroll
-    for (int v = 0; v < V; v++) out[v * TW + l] = extrap_smem<A, D, N>(sUnew, o, f, v, l, V);
-  }
-}
-
-template <typename T, typename A, int D, int N>
-__device__ __forceinline__ void extrap_next_tile(const Args<T, A> &a, int64_t tile, const A *sUnew, const SOps<A, N> &o)
-{
-  extrap_next_tile<T, A, D, N>(a, tile, sUnew, o, threadIdx.x, blockDim.x);
-}
-
-// ---------------------------------------------------------------------------
-// Euler: volume flux, common flux and divergence of one tile in one kernel.
-// ---------------------------------------------------------------------------
-template <typename T, typename A, int D, int N>
-__device__ __forceinline__ void euler_tile(const Args<T, A> &a, const LineOpsT<A, N> &ops, int64_t tile,
-                                           unsigned char *smem_raw, int tid, int nth, int bar)
-{
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, NM = G::NM;
-  A *sU = reinterpret_cast<A *>(smem_raw);
-  A *sF = sU + S * V * TW;
-  A *sFc = sF + D * S * V * TW;
-  A *sops = sFc + Fp * V * TW;
-  load_ops<A, N>(sops, ops, tid, nth);
-  {
-    const T *src = a.U + tile * (int64_t)S * V * TW;
-    for (int i = tid; i < S * V * TW; i += nth) sU[i] = src[i];
-  }
-  group_sync(bar, nth);
-  SOps<A, N> o(sops);
-  // transformed volume flux F~ = adj F (src/elements.cpp:1588-1699)
-  for (int it = tid; it < S * TW; it += nth)
-  {
-    const int s = it / TW, l = it % TW;
-    A U[V], F[V][D], P, Pp;
-#pragma unroll
-    for (int v = 0; v < V; v++) U[v] = sU[(s * V + v) * TW + l];
-    flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
-    const T *m = a.mets + (tile * S + s) * (int64_t)NM * TW + l;
-    A adj[D][D];
-#pragma unroll
-    for (int d1 = 0; d1 < D; d1++)
-#pragma unroll
-      for (int d2 = 0; d2 < D; d2++) adj[d1][d2] = m[(d1 * D + d2) * TW];
-#pragma unroll
-    for (int v = 0; v < V; v++)
-#pragma unroll
-      for (int d1 = 0; d1 < D; d1++)
-      {
-        A t = F[v][0] * adj[d1][0];
-#pragma unroll
-        for (int d2 = 1; d2 < D; d2++) t += F[v][d2] * adj[d1][d2];
-        sF[((d1 * S + s) * V + v) * TW + l] = t;
-      }
-  }
-  // common flux at the tile's flux points
-  for (int it = tid; it < Fp * TW; it += nth)
-  {
-    const int f = it / TW, l = it % TW;
-    const int64_t fi = (tile * Fp + f) * (int64_t)TW + l;
-    const int code = a.nbr[fi];
-    A n[D], dA;
-    const T *g = a.fgeo + (tile * Fp + f) * (int64_t)(D + 1) * TW + l;
-#pragma unroll
-    for (int d = 0; d < D; d++) n[d] = g[d * TW];
-    dA = g[D * TW];
-    A Uo[V], Un[V], UL[V], UR[V], UB[V], Fc[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) Uo[v] = uo[v * TW];
-    if (code >= 0) gather_fpt<T, A, V>(a.Ufp, code >> 1, Un);
-    conv_common<T, A, D>(a, Uo, Un, code, n, UL, UR, UB, Fc);
-    const bool right = (code >= 0) && (code & 1);
-#pragma unroll
-    for (int v = 0; v < V; v++) sFc[(f * V + v) * TW + l] = right ? -Fc[v] * dA : Fc[v] * dA;
-  }
-  group_sync(bar, nth);
-  for (int it = tid; it < S * TW; it += nth)
-  {
-    const int s = it / TW, l = it % TW;
-    A vol[V];
-#pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = A(0);
-#pragma unroll
-    for (int d = 0; d < D; d++)
-    {
-      int i, fm, fp;
-      spt_ends<D, N>(s, d, i, fm, fp);
-      const int st = pow_n<N>(d);
-      const int b = s - i * st;
-#pragma unroll
-      for (int m = 0; m < N; m++)
-      {
-        const A c = o.Dm[i * N + m];
-#pragma unroll
-        for (int v = 0; v < V; v++) vol[v] += c * sF[((d * S + b + m * st) * V + v) * TW + l];
-      }
-    }
-    finish_point<T, A, D, N>(a, tile, s, l, vol, sFc, o, a.extrap_next ? sU : nullptr);
-  }
-  if (a.extrap_next)
-  {
-    group_sync(bar, nth);
-    extrap_next_tile<T, A, D, N>(a, tile, sU, o, tid, nth);
-  }
-}
-
-
-// Shared memory of euler_tile (elements of the arithmetic type)
-template <int D, int N>
-constexpr int euler_smem_elems()
-{
-  return (Shape<D, N>::S * Shape<D, N>::V * (1 + D) + Shape<D, N>::Fp * Shape<D, N>::V) * TW + N * N + 4 * N;
-}
-
-template <typename T, typename A, int D, int N>
-__global__ void __launch_bounds__(Shape<D, N>::NT) k_euler(const __grid_constant__ Args<T, A> a,
-                                                                   const __grid_constant__ LineOpsT<A, N> ops)
-{
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  euler_tile<T, A, D, N>(a, ops, tile, smem_raw, threadIdx.x, blockDim.x, 0);
-}
-
-// ---------------------------------------------------------------------------
-// Navier-Stokes kernel 1: common solution, corrected gradient, viscous normal
-// flux at own flux points, volume flux and its divergence
-// (src/solver.cpp:1540-1600; src/elements.cpp:1393-1447, 1588-1699;
-//  src/faces.cpp:1366-1474, 508-710).
-// ---------------------------------------------------------------------------
-template <typename T, typename A, int D, int N>
-__global__ void __launch_bounds__(Shape<D, N>::NT, (D == 3) ? 2 : 1) k_ns_grad(const __grid_constant__ Args<T, A> a,
-                                                                                       const __grid_constant__ LineOpsT<A, N> ops)
-{
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, NM = G::NM;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  A *sU = reinterpret_cast<A *>(smem_raw);
-  A *sUC = sU + S * V * TW;
-  A *sdU = sUC + Fp * V * TW;  // [D][S][V][TW]: physical gradient, then F~
-  A *sops = sdU + D * S * V * TW;
-  load_ops<A, N>(sops, ops);
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  {
-    const T *src = a.U + tile * (int64_t)S * V * TW;
-    for (int i = threadIdx.x; i < S * V * TW; i += blockDim.x) sU[i] = src[i];
-  }
-  __syncthreads();
-  SOps<A, N> o(sops);
-  const A beta = a.ph.ldg_b;
-  // common solution at own flux points (LDG, flip_beta = 1)
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    const int64_t fi = (tile * Fp + f) * (int64_t)TW + l;
-    const int code = a.nbr[fi];
-    A Uo[V], UC[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) Uo[v] = uo[v * TW];
-    if (code >= 0)
-    {
-      A Un[V];
-      gather_fpt<T, A, V>(a.Ufp, code >> 1, Un);
-      const int slot = code & 1;
-#pragma unroll
-      for (int v = 0; v < V; v++)
-      {
-        const A ul = slot ? Un[v] : Uo[v];
-        const A ur = slot ? Uo[v] : Un[v];
-        if (beta == A(0.5))
-          UC[v] = ur;
-        else if (beta == A(-0.5))
-          UC[v] = ul;
-        else
-          UC[v] = A(0.5) * (ul + ur) - beta * (ul - ur);
-      }
-    }
-    else
-    {
-      A n[D], Ua[V], URa[V], UBa[V];
-      const T *g = a.fgeo + (tile * Fp + f) * (int64_t)(D + 1) * TW + l;
-#pragma unroll
-      for (int d = 0; d < D; d++) n[d] = g[d * TW];
-      to_abs<A, D>(Uo, Ua, a.ph);
-      ghost_state<A, D>(-code - 1, Ua, n, URa, UBa, a.ph);
-      to_stored<A, D>(UBa, UC, a.ph);
-    }
-#pragma unroll
-    for (int v = 0; v < V; v++) sUC[(f * V + v) * TW + l] = UC[v];
-  }
-  __syncthreads();
-  // corrected reference gradient, transformed to physical space
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A tdU[V][D];
-#pragma unroll
-    for (int d = 0; d < D; d++)
-    {
-      int i, fm, fp;
-      spt_ends<D, N>(s, d, i, fm, fp);
-      const int st = pow_n<N>(d);
-      const int b = s - i * st;
-#pragma unroll
-      for (int v = 0; v < V; v++)
-      {
-        A acc = A(0);
-#pragma unroll
-        for (int m = 0; m < N; m++) acc += o.Dm[i * N + m] * sU[((b + m * st) * V + v) * TW + l];
-        const A cm = o.Dbm[i] * sUC[(fm * V + v) * TW + l];
-        const A cp = o.Dbp[i] * sUC[(fp * V + v) * TW + l];
-        tdU[v][d] = acc + ((fm < fp) ? (cm + cp) : (cp + cm));
-      }
-    }
-    const T *m = a.mets + (tile * S + s) * (int64_t)NM * TW + l;
-    A adj[D][D];
-#pragma unroll
-    for (int d1 = 0; d1 < D; d1++)
-#pragma unroll
-      for (int d2 = 0; d2 < D; d2++) adj[d1][d2] = m[(d1 * D + d2) * TW];
-    const A inv_det = A(1) / m[D * D * TW];
-#pragma unroll
-    for (int v = 0; v < V; v++)
-#pragma unroll
-      for (int d1 = 0; d1 < D; d1++)
-      {
-        A g = tdU[v][0] * adj[0][d1];
-#pragma unroll
-        for (int d2 = 1; d2 < D; d2++) g += tdU[v][d2] * adj[d2][d1];
-        sdU[((d1 * S + s) * V + v) * TW + l] = g * inv_det;
-      }
-  }
-  __syncthreads();
-  if (a.dU_out)
-  {
-    T *g = a.dU_out + tile * (int64_t)D * S * V * TW;
-    for (int i = threadIdx.x; i < D * S * V * TW; i += blockDim.x) g[i] = (T)sdU[i];
-  }
-  // viscous normal flux at own flux points (own side; boundaries: prescribed side)
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    const int64_t fi = (tile * Fp + f) * (int64_t)TW + l;
-    const int code = a.nbr[fi];
-    if (code >= 0 && ((beta == A(0.5) && (code & 1)) || (beta == A(-0.5) && !(code & 1)))) continue;
-    A n[D];
-    const T *g = a.fgeo + (tile * Fp + f) * (int64_t)(D + 1) * TW + l;
-#pragma unroll
-    for (int d = 0; d < D; d++) n[d] = g[d * TW];
-    A Uf[V], dUf[V][D], Fn[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++)
-    {
-      Uf[v] = uo[v * TW];
-#pragma unroll
-      for (int d = 0; d < D; d++) dUf[v][d] = extrap_smem<A, D, N>(sdU + d * S * V * TW, o, f, v, l, V);
-    }
-    A Ua[V];
-    to_abs<A, D>(Uf, Ua, a.ph);
-    if (code >= 0)
-      visc_normal<A, D>(Ua, dUf, n, Fn, a.ph);
-    else
-    {
-      A UB[V], dUB[V][D];
-      if constexpr (Pert<A>::on)
-      {
-        A UR[V];
-        ghost_state<A, D>(-code - 1, Ua, n, UR, UB, a.ph);
-      }
-      else
-      {
-        // the prescribed state is the point's common solution
-#pragma unroll
-        for (int v = 0; v < V; v++) UB[v] = sUC[(f * V + v) * TW + l];
-      }
-      ghost_grad<A, D>(-code - 1, Ua, dUf, n, dUB);
-      visc_normal<A, D>(UB, dUB, n, Fn, a.ph);
-    }
-    T *out = a.Fvn + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) out[v * TW] = Fn[v];
-  }
-  __syncthreads();
-  // flux at solution points, transformed: F~ = adj (F_conv + F_visc)
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A U[V], dU[V][D], F[V][D];
-#pragma unroll
-    for (int v = 0; v < V; v++)
-    {
-      U[v] = sU[(s * V + v) * TW + l];
-#pragma unroll
-      for (int d = 0; d < D; d++) dU[v][d] = sdU[((d * S + s) * V + v) * TW + l];
-    }
-    A P, Pp, Ua[V];
-    flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
-    to_abs<A, D>(U, Ua, a.ph);
-    flux_visc_add<A, D>(Ua, dU, F, a.ph);
-    const T *m = a.mets + (tile * S + s) * (int64_t)NM * TW + l;
-    A adj[D][D];
-#pragma unroll
-    for (int d1 = 0; d1 < D; d1++)
-#pragma unroll
-      for (int d2 = 0; d2 < D; d2++) adj[d1][d2] = m[(d1 * D + d2) * TW];
-#pragma unroll
-    for (int v = 0; v < V; v++)
-#pragma unroll
-      for (int d1 = 0; d1 < D; d1++)
-      {
-        A t = F[v][0] * adj[d1][0];
-#pragma unroll
-        for (int d2 = 1; d2 < D; d2++) t += F[v][d2] * adj[d1][d2];
-        sdU[((d1 * S + s) * V + v) * TW + l] = t;
-      }
-  }
-  __syncthreads();
-  // volume divergence
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A vol[V];
-#pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = A(0);
-#pragma unroll
-    for (int d = 0; d < D; d++)
-    {
-      int i, fm, fp;
-      spt_ends<D, N>(s, d, i, fm, fp);
-      const int st = pow_n<N>(d);
-      const int b = s - i * st;
-#pragma unroll
-      for (int m = 0; m < N; m++)
-      {
-        const A c = o.Dm[i * N + m];
-#pragma unroll
-        for (int v = 0; v < V; v++) vol[v] += c * sdU[((d * S + b + m * st) * V + v) * TW + l];
-      }
-    }
-    A *out = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) out[v * TW] = vol[v];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Navier-Stokes kernel 2: convective + LDG common flux, surface correction,
-// optional RK update (src/faces.cpp:1476-1614; src/elements.cpp:1476-1501).
-// ---------------------------------------------------------------------------
-template <typename T, typename A, int D, int N>
-__global__ void __launch_bounds__(Shape<D, N>::NT) k_ns_face(const __grid_constant__ Args<T, A> a,
-                                                                     const __grid_constant__ LineOpsT<A, N> ops)
-{
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  A *sFc = reinterpret_cast<A *>(smem_raw);
-  A *sUnew = sFc + Fp * V * TW;
-  A *sops = sUnew + S * V * TW;
-  load_ops<A, N>(sops, ops);
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  __syncthreads();
-  SOps<A, N> o(sops);
-  const A beta = a.ph.ldg_b, tau = a.ph.ldg_tau;
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    const int64_t fi = (tile * Fp + f) * (int64_t)TW + l;
-    const int code = a.nbr[fi];
-    A n[D], dA;
-    const T *g = a.fgeo + (tile * Fp + f) * (int64_t)(D + 1) * TW + l;
-#pragma unroll
-    for (int d = 0; d < D; d++) n[d] = g[d * TW];
-    dA = g[D * TW];
-    A Uo[V], Un[V], UL[V], UR[V], UB[V], Fc[V], Fv[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) Uo[v] = uo[v * TW];
-    if (code >= 0) gather_fpt<T, A, V>(a.Ufp, code >> 1, Un);
-    conv_common<T, A, D>(a, Uo, Un, code, n, UL, UR, UB, Fc);
-    const T *fvo = a.Fvn + (tile * Fp + f) * (int64_t)V * TW + l;
-    if (code >= 0)
-    {
-      const int slot = code & 1;
-      A FnL[V], FnR[V];
-      // own side is left when slot == 0
-      if (beta == A(0.5))
-      {
-        if (slot == 0)
-        {
-#pragma unroll
-          for (int v = 0; v < V; v++) FnL[v] = fvo[v * TW];
-        }
-        else
-          gather_fpt<T, A, V>(a.Fvn, code >> 1, FnL);
-#pragma unroll
-        for (int v = 0; v < V; v++) FnR[v] = A(0);
-      }
-      else if (beta == A(-0.5))
-      {
-        if (slot == 1)
-        {
-#pragma unroll
-          for (int v = 0; v < V; v++) FnR[v] = fvo[v * TW];
-        }
-        else
-          gather_fpt<T, A, V>(a.Fvn, code >> 1, FnR);
-#pragma unroll
-        for (int v = 0; v < V; v++) FnL[v] = A(0);
-      }
-      else
-      {
-        A Fo[V], Fx[V];
-#pragma unroll
-        for (int v = 0; v < V; v++) Fo[v] = fvo[v * TW];
-        gather_fpt<T, A, V>(a.Fvn, code >> 1, Fx);
-#pragma unroll
-        for (int v = 0; v < V; v++)
-        {
-          FnL[v] = slot ? Fx[v] : Fo[v];
-          FnR[v] = slot ? Fo[v] : Fx[v];
-        }
-      }
-#pragma unroll
-      for (int v = 0; v < V; v++)
-        Fv[v] = A(0.5) * (FnL[v] + FnR[v]) + tau * (UL[v] - UR[v]) + beta * (FnL[v] - FnR[v]);
-    }
-    else
-    {
-#pragma unroll
-      for (int v = 0; v < V; v++) Fv[v] = fvo[v * TW] + tau * (UL[v] - UB[v]);
-    }
-    const bool right = (code >= 0) && (code & 1);
-#pragma unroll
-    for (int v = 0; v < V; v++)
-    {
-      A acc = right ? -Fc[v] * dA : Fc[v] * dA;
-      if (right)
-        acc -= Fv[v] * dA;
-      else
-        acc += Fv[v] * dA;
-      sFc[(f * V + v) * TW + l] = acc;
-    }
-  }
-  __syncthreads();
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A vol[V];
-    const A *dv = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = dv[v * TW];
-    finish_point<T, A, D, N>(a, tile, s, l, vol, sFc, o, a.extrap_next ? sUnew : nullptr);
-  }
-  if (a.extrap_next)
-  {
-    __syncthreads();
-    extrap_next_tile<T, A, D, N>(a, tile, sUnew, o);
+    a.Uout[idx] = u;
+    unew[v] = (A)(T)u;
   }
 }
 

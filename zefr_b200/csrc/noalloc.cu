@@ -18,6 +18,7 @@
 
 #include "ctx_impl.cuh"
 #include "hex_kernels.cuh"
+#include "quad_kernels.cuh"
 
 namespace zb {
 namespace {
@@ -208,7 +209,7 @@ template <int D, int N>
 void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStream_t st)
 {
   using G = dev::Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, NT = G::NT;
+  [[maybe_unused]] constexpr int S = G::S, Fp = G::Fp, V = G::V;
   const auto ops = line_ops_d<N>(p);
   dev::Args<double, double> a;
   std::memset(&a, 0, sizeof(a));
@@ -257,29 +258,31 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
       dev::k_hex_ns_face<double, double, N><<<(unsigned)p.ntiles, HT * ZF, smem2, st>>>(a, ops);
       NA_CK(cudaGetLastError());
     }
-    return;
-  }
-  dev::k_extrap<double, double, D, N><<<blocks_for(p.ntiles * Fp * TW), 256, 0, st>>>(
-      a.U, reinterpret_cast<double *>(base + r.Ufp), p.ntiles, ops);
-  NA_CK(cudaGetLastError());
-  const size_t ob = sizeof(dev::LineOpsT<double, N>);
-  if (!p.params.viscous)
-  {
-    const size_t smem = (size_t)(S * V + D * S * V + Fp * V) * TW * sizeof(double) + ob;
-    NA_CK(cudaFuncSetAttribute(dev::k_euler<double, double, D, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dev::k_euler<double, double, D, N><<<(unsigned)p.ntiles, NT, smem, st>>>(a, ops);
-    NA_CK(cudaGetLastError());
   }
   else
   {
-    const size_t smem1 = (size_t)(S * V + Fp * V + D * S * V) * TW * sizeof(double) + ob;
-    NA_CK(cudaFuncSetAttribute(dev::k_ns_grad<double, double, D, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
-    dev::k_ns_grad<double, double, D, N><<<(unsigned)p.ntiles, NT, smem1, st>>>(a, ops);
+    constexpr int NT = dev::QuadShape<N>::NT;
+    dev::k_extrap<double, double, N><<<blocks_for(p.ntiles * Fp * TW), 256, 0, st>>>(
+        a.U, reinterpret_cast<double *>(base + r.Ufp), p.ntiles, ops);
     NA_CK(cudaGetLastError());
-    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(double) + ob;
-    NA_CK(cudaFuncSetAttribute(dev::k_ns_face<double, double, D, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-    dev::k_ns_face<double, double, D, N><<<(unsigned)p.ntiles, NT, smem2, st>>>(a, ops);
-    NA_CK(cudaGetLastError());
+    if (!p.params.viscous)
+    {
+      const size_t smem = dev::euler_smem_elems<N>() * sizeof(double);
+      NA_CK(cudaFuncSetAttribute(dev::k_euler<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      dev::k_euler<double, double, N><<<(unsigned)p.ntiles, NT, smem, st>>>(a, ops);
+      NA_CK(cudaGetLastError());
+    }
+    else
+    {
+      const size_t smem1 = dev::quad_grad_smem_elems<N>() * sizeof(double);
+      NA_CK(cudaFuncSetAttribute(dev::k_ns_grad<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+      dev::k_ns_grad<double, double, N><<<(unsigned)p.ntiles, NT, smem1, st>>>(a, ops);
+      NA_CK(cudaGetLastError());
+      const size_t smem2 = dev::quad_face_smem_elems<N>() * sizeof(double);
+      NA_CK(cudaFuncSetAttribute(dev::k_ns_face<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+      dev::k_ns_face<double, double, N><<<(unsigned)p.ntiles, NT, smem2, st>>>(a, ops);
+      NA_CK(cudaGetLastError());
+    }
   }
 }
 

@@ -1,5 +1,6 @@
 // Launches of the quadrilateral residual kernels.
 #include "ctx_impl.cuh"
+#include "quad_kernels.cuh"
 #include "time_kernels.cuh"
 
 namespace zb {
@@ -7,9 +8,9 @@ namespace zb {
 template <typename T, typename A, int N>
 static void launch_extrap_quad(Ctx &c)
 {
-  const int64_t work = c.ntiles * Shape<2, N>::Fp * TW;
+  const int64_t work = c.ntiles * dev::QuadShape<N>::Fp * TW;
   ProfScope ps(c, ZB_K_EXTRAP);
-  dev::k_extrap<T, A, 2, N><<<grid_for(work, 256), 256, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles,
+  dev::k_extrap<T, A, N><<<grid_for(work, 256), 256, 0, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles,
                                                                        line_ops<A, N>(c.plan));
   c.launches++;
   CK(cudaGetLastError());
@@ -18,37 +19,34 @@ static void launch_extrap_quad(Ctx &c)
 template <typename T, typename A, int N>
 static void launch_stage_quad(Ctx &c, const StageCfg &sc)
 {
-  constexpr int D = 2;
-  using G = Shape<D, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, NT = G::NT;
+  constexpr int NT = dev::QuadShape<N>::NT;
   const Args<T, A> a = make_args<T, A>(c, sc);
   const LineOpsT<A, N> ops = line_ops<A, N>(c.plan);
-  const size_t ops_bytes = sizeof(LineOpsT<A, N>);
   if (!c.plan.params.viscous)
   {
-    const size_t smem = (size_t)(S * V + D * S * V + Fp * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_euler<T, A, D, N>, smem);
+    const size_t smem = dev::euler_smem_elems<N>() * sizeof(A);
+    set_smem(dev::k_euler<T, A, N>, smem);
     ProfScope ps(c, ZB_K_EULER);
-    dev::k_euler<T, A, D, N><<<(unsigned)c.ntiles, NT, smem, c.stream>>>(a, ops);
+    dev::k_euler<T, A, N><<<(unsigned)c.ntiles, NT, smem, c.stream>>>(a, ops);
     c.launches++;
     CK(cudaGetLastError());
   }
   else
   {
-    const size_t smem1 = (size_t)(S * V + Fp * V + D * S * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_ns_grad<T, A, D, N>, smem1);
+    const size_t smem1 = dev::quad_grad_smem_elems<N>() * sizeof(A);
+    set_smem(dev::k_ns_grad<T, A, N>, smem1);
     if (!sc.face_only)
     {
       ProfScope ps(c, ZB_K_NS_GRAD);
-      dev::k_ns_grad<T, A, D, N><<<(unsigned)c.ntiles, NT, smem1, c.stream>>>(a, ops);
+      dev::k_ns_grad<T, A, N><<<(unsigned)c.ntiles, NT, smem1, c.stream>>>(a, ops);
       c.launches++;
       CK(cudaGetLastError());
     }
     if (sc.grad_only) return;
-    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A) + ops_bytes;
-    set_smem(dev::k_ns_face<T, A, D, N>, smem2);
+    const size_t smem2 = dev::quad_face_smem_elems<N>() * sizeof(A);
+    set_smem(dev::k_ns_face<T, A, N>, smem2);
     ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_ns_face<T, A, D, N><<<(unsigned)c.ntiles, NT, smem2, c.stream>>>(a, ops);
+    dev::k_ns_face<T, A, N><<<(unsigned)c.ntiles, NT, smem2, c.stream>>>(a, ops);
     c.launches++;
     CK(cudaGetLastError());
   }

@@ -40,7 +40,7 @@ static void launch_stage_tri(Ctx &c, const StageCfg &sc)
   }
   else
   {
-    const size_t smem1 = (ops + (size_t)(S * V + Fp * V + D * S * V) * TW) * sizeof(A);
+    const size_t smem1 = (ops + (size_t)(S * V + Fp * V + 2 * D * S * V) * TW) * sizeof(A);
     if (!sc.face_only)
     {
       ProfScope ps(c, ZB_K_NS_GRAD);

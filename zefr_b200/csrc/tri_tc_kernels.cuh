@@ -364,7 +364,9 @@ __global__ void __launch_bounds__(TriTc<N>::NT) k_tri_ns_grad_tc(const __grid_co
     flux_conv_stored<float, D>(U, F, P, Pp, a.ph);
     to_abs<float, D>(U, Ua, a.ph);
     flux_visc_add<float, D>(Ua, dU, F, a.ph);
-    tri_transform<float, float>(a, tile, s, ll, F, sdU + qq * C::TILE_DU, S);
+    const float *m = a.mets + (tile * S + s) * (int64_t)5 * TW + ll;
+    const float adj[2][2] = {{m[0], m[TW]}, {m[2 * TW], m[3 * TW]}};
+    tri_transform<float>(F, adj, sdU + qq * C::TILE_DU, S, s, ll);
   }
   __syncthreads();
   // ---- product 3: volume divergence ----------------------------------------
