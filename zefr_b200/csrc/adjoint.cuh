@@ -1279,8 +1279,21 @@ __device__ __forceinline__ void face_item(int it, int &f, int &l)
   l = rest % TW;
 }
 
+// Quadrilaterals hold the state adjoint's pass to 512 threads per SM (128
+// registers, some 800 bytes of the boundary path spilled): 240 registers left
+// two 128-thread CTAs, and the pass waits on its own dependent arithmetic.
+// P3 200^2 Roe 148 -> 122 us at three CTAs (168 registers) and at four, Rusanov
+// 149 -> 122 -> 117, the 48 x 96 cylinder 74 -> 75 -> 68.  Hexahedra stay at one
+// 256-thread CTA beside 223 KB of shared memory: 384 threads of 168 registers
+// 404 -> 456 us (24^3 P3), 512 of 128 502.
 template <int D, int N, bool GEO>
-__global__ void __launch_bounds__(Shape<D, N>::NT) k_adj_ns1(const __grid_constant__ AdjArgs a,
+constexpr int adj_ns1_minb()
+{
+  return D == 2 && !GEO ? 512 / Shape<D, N>::NT : 1;
+}
+
+template <int D, int N, bool GEO>
+__global__ void __launch_bounds__(Shape<D, N>::NT, adj_ns1_minb<D, N, GEO>()) k_adj_ns1(const __grid_constant__ AdjArgs a,
                                                                            const __grid_constant__ LineOpsT<double, N> ops)
 {
   using G = Shape<D, N>;
