@@ -32,7 +32,7 @@ static void launch_adj_kernels(Ctx &c, const dev::AdjArgs &a, const LineOpsT<dou
   }
   // the state adjoint's staged face inputs: [Fp][3V + D][TW]
   const size_t smem1 = (size_t)(GEO ? 2 * S * V + Fp * V + 2 * D * S * V
-                                    : S * V + Fp * V + D * S * V + Fp * (3 * V + D)) *
+                                    : S * V + dev::adj_ns1_uc_points<D, N, false>() * V + D * S * V + Fp * (3 * V + D)) *
                        TW * sizeof(double);
   set_smem(dev::k_adj_ns1<D, N, GEO>, smem1);
   {

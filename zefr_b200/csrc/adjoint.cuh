@@ -1279,6 +1279,15 @@ __device__ __forceinline__ void face_item(int it, int &f, int &l)
   l = rest % TW;
 }
 
+// Points of the common-solution array of k_adj_ns1: the state adjoint reuses it
+// for the volume part [S][V][TW], which outgrows the flux points of
+// quadrilaterals from P4 on (N^2 > 4 N)
+template <int D, int N, bool GEO>
+constexpr int adj_ns1_uc_points()
+{
+  return !GEO && Shape<D, N>::S > Shape<D, N>::Fp ? Shape<D, N>::S : Shape<D, N>::Fp;
+}
+
 // Quadrilaterals hold the state adjoint's pass to 512 threads per SM (128
 // registers, some 800 bytes of the boundary path spilled): 240 registers left
 // two 128-thread CTAs, and the pass waits on its own dependent arithmetic.
@@ -1300,8 +1309,8 @@ __global__ void __launch_bounds__(Shape<D, N>::NT, adj_ns1_minb<D, N, GEO>()) k_
   constexpr int S = G::S, Fp = G::Fp, V = G::V, NM = G::NM;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *sU = reinterpret_cast<double *>(smem_raw);  // [S][V][TW]
-  double *sUC = sU + S * V * TW;                       // [Fp][V][TW]
-  double *sdU = sUC + Fp * V * TW;                     // [D][S][V][TW] physical gradient
+  double *sUC = sU + S * V * TW;                       // [Fp][V][TW], reused below
+  double *sdU = sUC + adj_ns1_uc_points<D, N, GEO>() * V * TW;  // [D][S][V][TW] physical gradient
   // The state adjoint reuses the common solution's array for the volume
   // flux's U adjoint [S][V][TW] and the gradient's for the gradient adjoint
   // [D][S][V][TW] (each dead by then), which leaves more of the SM's L1 to
