@@ -1101,11 +1101,13 @@ static void ensure_adjoint_buffers(Ctx *c)
 // tiles on the host) and the geometry adjoint (c->mbar / c->gbar, added to
 // the device sums with `accumulate`).  The geometry adjoint of the viscous
 // form reads this state's forward viscous normal flux from c->Fvn: computed
-// here unless `fvn_ready` says the caller has put it there.
-static void vjp_tiles(Ctx *c, bool params, double *param_bar, bool geo, bool accumulate, bool fvn_ready = false)
+// here unless `fvn_ready` says the caller has put it there.  `traces_ready`:
+// the trace buffer holds the current state's traces where ufp_valid says so.
+static void vjp_tiles(Ctx *c, bool params, double *param_bar, bool geo, bool accumulate, bool fvn_ready = false,
+                      bool traces_ready = false)
 {
   // linearisation point: the current state and its traces
-  c->ufp_valid = false;
+  if (!traces_ready) c->ufp_valid = false;
   ensure_ufp(c);
   const int NM = c->D * c->D + 1;
   if (geo)
@@ -1176,25 +1178,14 @@ void ctx_vjp(Ctx *c, const double *lam, double *Ubar, int64_t ss, int64_t vs, in
 // reverse of one RK44 step (tile layout, FP64)
 // ---------------------------------------------------------------------------
 
-// out = a - (c * (1/|J|)) * r per point (the RK stage update)
-__global__ void k_stage_state(double *__restrict__ out, const double *__restrict__ a, const double *__restrict__ r,
-                              const double *__restrict__ mets, double c, int64_t ntiles, int S, int V, int NM, int DD)
-{
-  const int64_t total = ntiles * S * V * TW;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
-  {
-    const int l = (int)(i % TW);
-    const int64_t ps = i / ((int64_t)TW * V);
-    const double inv = 1.0 / mets[(ps * NM + DD) * TW + l];
-    out[i] = a[i] - c * inv * r[i];
-  }
-}
-
 // lam = cb * (1/|J|) * ubar1 [+ ca * (1/|J|) * ubs]: the stage residual's
-// adjoint weight (cb = -b_s dt, ca = -a_s dt)
+// adjoint weight (cb = -b_s dt, ca = -a_s dt).  With a later stage's adjoint
+// ubs also the running result: ub0 = base + ubs (base: ubar1 the first time,
+// then ub0 itself).
 __global__ void k_stage_weight(double *__restrict__ lam, const double *__restrict__ ubar1,
-                               const double *__restrict__ ubs, const double *__restrict__ mets, double cb, double ca,
-                               int64_t ntiles, int S, int V, int NM, int DD)
+                               const double *__restrict__ ubs, const double *base, double *ub0,
+                               const double *__restrict__ mets, double cb, double ca, int64_t ntiles, int S, int V,
+                               int NM, int DD)
 {
   const int64_t total = ntiles * S * V * TW;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
@@ -1203,7 +1194,11 @@ __global__ void k_stage_weight(double *__restrict__ lam, const double *__restric
     const int64_t ps = i / ((int64_t)TW * V);
     const double inv = 1.0 / mets[(ps * NM + DD) * TW + l];
     double w = cb * inv * ubar1[i];
-    if (ubs) w = w + ca * inv * ubs[i];
+    if (ubs)
+    {
+      w = w + ca * inv * ubs[i];
+      ub0[i] = base[i] + ubs[i];
+    }
     lam[i] = w;
   }
 }
@@ -1233,6 +1228,39 @@ __global__ void k_add(double *__restrict__ a, const double *__restrict__ b, int6
     a[i] += b[i];
 }
 
+// sum of the four stages' free-stream adjoints per tile, last stage first
+__global__ void k_sum_stages(double *__restrict__ out, const double *__restrict__ p, int64_t n)
+{
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = ((p[3 * n + i] + p[2 * n + i]) + p[n + i]) + p[i];
+}
+
+// Points the context's state, RK start state, residual registers, viscous
+// normal flux and adjoint outputs at other buffers for a while: a launch takes
+// its pointers by value, so the stages of the step adjoint work in their own
+// arrays and nothing is copied to and from the context's.
+struct BufferScope
+{
+  Ctx &c;
+  void *U, *U_ini, *divF[4], *Fvn;
+  double *Ubar, *pbar;
+  explicit BufferScope(Ctx &cc) : c(cc), U(cc.U), U_ini(cc.U_ini), Fvn(cc.Fvn), Ubar(cc.Ubar), pbar(cc.pbar)
+  {
+    for (int s = 0; s < 4; s++) divF[s] = cc.divF[s];
+  }
+  ~BufferScope()
+  {
+    c.U = U;
+    c.U_ini = U_ini;
+    c.Fvn = Fvn;
+    c.Ubar = Ubar;
+    c.pbar = pbar;
+    for (int s = 0; s < 4; s++) c.divF[s] = divF[s];
+    c.ufp_valid = false;
+    c.need_fvn = false;
+  }
+};
+
 void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar0, int64_t ss, int64_t vs,
                      int64_t es, int where, double *param_bar, bool geometry)
 {
@@ -1248,10 +1276,11 @@ void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar
   {
     // stage states 0..3, stage residuals 0..3, the end state's adjoint, one
     // stage adjoint and the running result, in the tile layout; the
-    // free-stream adjoint per tile summed over the stages
-    c->rkv = (double *)dalloc(((size_t)11 * nU + (size_t)c->ntiles * 5) * sizeof(double));
+    // free-stream adjoint per tile of each stage and its sum
+    c->rkv = (double *)dalloc(((size_t)11 * nU + (size_t)c->ntiles * 5 * 5) * sizeof(double));
   }
-  double *pb_acc = c->rkv + (size_t)11 * nU;
+  const int64_t np = c->ntiles * 5;
+  double *pb = c->rkv + (size_t)11 * nU, *pb_sum = pb + 4 * np;
   // the geometry adjoint of the viscous form needs each stage's forward
   // viscous normal flux: kept from the forward sweep
   const bool keep_fvn = geometry && c->plan.params.viscous;
@@ -1273,52 +1302,39 @@ void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar
     src = stage_in(c, Ubar1, ext, where);
     to_tiles<double>(c, src, ub1, nullptr, nullptr, ss, vs, es);
   }
-  // forward: the stage states and residuals (FRSolver::step_RK's stages)
+  BufferScope scope(*c);
+  for (int s = 0; s < 4; s++) c->divF[s] = Rs[s];
+  c->U_ini = Us[0];
+  // forward: the stage states and residuals (FRSolver::step_RK's stages); the
+  // stage kernels' RK update writes the next stage's state and traces
+  c->ufp_valid = false;
   for (int s = 0; s < 4; s++)
   {
-    CK(cudaMemcpyAsync(c->U, Us[s], (size_t)nU * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    c->ufp_valid = false;
-    ensure_ufp(c);
-    StageCfg sc{0, 0, 0, 0};
+    c->U = Us[s];
+    if (keep_fvn) c->Fvn = c->rkfvn + s * nF;
+    ensure_stage_ufp(c);
+    StageCfg sc{(unsigned)s, s < 3 ? 1 : 0, 0, s < 3 ? 1 : 0};
+    if (s < 3) sc.Uout = Us[s + 1];
     c->need_fvn = keep_fvn;
     c->launch_stage(*c, sc);
     c->need_fvn = false;
-    CK(cudaMemcpyAsync(Rs[s], c->divF[0], (size_t)nU * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    if (keep_fvn)
-      CK(cudaMemcpyAsync(c->rkfvn + s * nF, c->Fvn, nF * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    if (s < 3)
-    {
-      k_stage_state<<<grid, 256, 0, c->stream>>>(Us[s + 1], Us[0], Rs[s], (const double *)c->mets, kRkAlpha[s] * dt,
-                                                 c->ntiles, S, V, NM, DD);
-      c->launches++;
-      CK(cudaGetLastError());
-    }
   }
   // reverse: Ubar0 = Ubar1 + sum_s (dR_s/dU_s)^T lam_s with the stage weights
-  // lam_s = -b_s dt/|J| Ubar1 - a_s dt/|J| Ubar_{s+1}
-  CK(cudaMemcpyAsync(ub0, ub1, (size_t)nU * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-  if (param_bar) CK(cudaMemsetAsync(pb_acc, 0, (size_t)c->ntiles * 5 * sizeof(double), c->stream));
+  // lam_s = -b_s dt/|J| Ubar1 - a_s dt/|J| Ubar_{s+1}; the stage adjoints
+  // alternate between two buffers
   for (int s = 3; s >= 0; s--)
   {
-    k_stage_weight<<<grid, 256, 0, c->stream>>>(c->lam, ub1, s < 3 ? ubs : nullptr, (const double *)c->mets,
-                                                -kRkBeta[s] * dt, s < 3 ? -kRkAlpha[s] * dt : 0.0, c->ntiles, S, V,
-                                                NM, DD);
+    const bool later = s < 3;
+    k_stage_weight<<<grid, 256, 0, c->stream>>>(c->lam, ub1, later ? ubs : nullptr, s == 2 ? ub1 : ub0, ub0,
+                                                (const double *)c->mets, -kRkBeta[s] * dt,
+                                                later ? -kRkAlpha[s] * dt : 0.0, c->ntiles, S, V, NM, DD);
     c->launches++;
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(c->U, Us[s], (size_t)nU * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    if (keep_fvn)
-      CK(cudaMemcpyAsync(c->Fvn, c->rkfvn + s * nF, nF * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    vjp_tiles(c, param_bar != nullptr, nullptr, geometry, geometry, keep_fvn);
-    if (param_bar)
-    {
-      k_accumulate<<<grid_for(c->ntiles * 5, 256), 256, 0, c->stream>>>(pb_acc, c->pbar, c->ntiles * 5);
-      c->launches++;
-      CK(cudaGetLastError());
-    }
-    CK(cudaMemcpyAsync(ubs, c->Ubar, (size_t)nU * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    k_add<<<grid, 256, 0, c->stream>>>(ub0, ubs, nU);
-    c->launches++;
-    CK(cudaGetLastError());
+    c->U = Us[s];
+    if (keep_fvn) c->Fvn = c->rkfvn + s * nF;
+    c->pbar = pb + s * np;
+    vjp_tiles(c, param_bar != nullptr, nullptr, geometry, geometry, keep_fvn, s == 3);
+    std::swap(c->Ubar, ubs);  // ubs: this stage's adjoint
     if (geometry && s > 0)
     {
       // U_s = U_0 - a_{s-1} dt R_{s-1} / |J|
@@ -1339,11 +1355,17 @@ void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar
       CK(cudaGetLastError());
     }
   }
+  k_add<<<grid, 256, 0, c->stream>>>(ub0, ubs, nU);
+  c->launches++;
+  CK(cudaGetLastError());
   if (param_bar)
   {
     // one read of the stage-summed tiles, summed over tiles in a fixed order
-    std::vector<double> h((size_t)c->ntiles * 5);
-    CK(cudaMemcpyAsync(h.data(), pb_acc, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    k_sum_stages<<<grid_for(np, 256), 256, 0, c->stream>>>(pb_sum, pb, np);
+    c->launches++;
+    CK(cudaGetLastError());
+    std::vector<double> h((size_t)np);
+    CK(cudaMemcpyAsync(h.data(), pb_sum, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     double pacc[5] = {0, 0, 0, 0, 0};
     for (int64_t t = 0; t < c->ntiles; t++)
@@ -1351,7 +1373,6 @@ void ctx_rk_step_vjp(Ctx *c, const double *U0, const double *Ubar1, double *Ubar
     for (int k = 0; k < 5; k++) param_bar[k] += pacc[k];
   }
   from_tiles(c, ub0, nullptr, nullptr, Ubar0, ss, vs, es, where);
-  c->ufp_valid = false;
 }
 
 void ctx_wall_force(Ctx *c, double *out)

@@ -33,6 +33,7 @@ struct StageCfg
   int want_dU = 0;     // write the physical gradient (NS)
   int grad_only = 0;   // NS: stop after the gradient kernel
   int face_only = 0;   // NS: the face kernel alone (the gradient kernel ran before)
+  void *Uout = nullptr;  // where the RK update writes (nullptr: in place)
 };
 
 // RK44 tables (src/solver.cpp:722-735)
@@ -260,7 +261,7 @@ static Args<T, A> make_args(Ctx &c, const StageCfg &sc)
   // the one-sided form keeps no trace buffer: the gradient kernel forms the
   // traces from the state, so the next stage's extrapolation is not stored
   a.extrap_next = a.Fcom ? 0 : sc.extrap_next;
-  a.Uout = (T *)c.U;
+  a.Uout = (T *)(sc.Uout ? sc.Uout : c.U);
   a.U_ini = (T *)c.U_ini;
   a.Ucomp = nullptr;
   a.dt = (A)c.dt;
