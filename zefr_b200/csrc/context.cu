@@ -529,6 +529,41 @@ static void upload_static(Ctx &c)
   CK(cudaStreamSynchronize(c.stream));
 }
 
+// The triangle operators as the kernels take them: oppE, oppD, oppD_fpts,
+// oppDiv, oppDiv_fpts back to back (TriShape), then each kernel's own block
+// (TriRun): gradient (oppD, oppD_fpts and oppDiv as pairs, oppE), face
+// (oppDiv_fpts, oppE), Euler (oppDiv as pairs, oppDiv_fpts, oppE).
+static std::vector<double> tri_operator_blocks(const Plan &p)
+{
+  const int S = p.nspts, Fp = p.nfpts;
+  std::vector<double> o;
+  const auto append = [&](const std::vector<double> &v) { o.insert(o.end(), v.begin(), v.end()); };
+  const auto pad = [&] { o.resize((o.size() + 3) / 4 * 4, 0.0); };
+  // rows x cols of both dimensions from src[d * dim_stride + row * row_stride + col]
+  const auto pairs = [&](const std::vector<double> &v, int cols, int row_stride, int dim_stride) {
+    for (int r = 0; r < S; r++)
+      for (int c = 0; c < cols; c++)
+        for (int d = 0; d < 2; d++) o.push_back(v[(size_t)d * dim_stride + (size_t)r * row_stride + c]);
+  };
+  for (const auto *v : {&p.tri_oppE, &p.tri_oppD, &p.tri_oppD_fpts, &p.tri_oppDiv, &p.tri_oppDiv_fpts}) append(*v);
+  pad();
+  pairs(p.tri_oppD, S, S, S * S);
+  pairs(p.tri_oppD_fpts, Fp, Fp, S * Fp);
+  pairs(p.tri_oppDiv, S, 2 * S, S);
+  append(p.tri_oppE);
+  pad();
+  append(p.tri_oppDiv_fpts);
+  pad();
+  append(p.tri_oppE);
+  pad();
+  pairs(p.tri_oppDiv, S, 2 * S, S);
+  append(p.tri_oppDiv_fpts);
+  pad();
+  append(p.tri_oppE);
+  pad();
+  return o;
+}
+
 Ctx *ctx_create(const Plan &plan)
 {
   std::unique_ptr<Ctx> c(new Ctx());
@@ -600,11 +635,7 @@ Ctx *ctx_create(const Plan &plan)
       upload_static<float>(*c);
     if (plan.etype == ET_TRI)
     {
-      // oppE, oppD, oppD_fpts, oppDiv, oppDiv_fpts back to back (TriShape)
-      std::vector<double> ops;
-      for (const auto *v : {&plan.tri_oppE, &plan.tri_oppD, &plan.tri_oppD_fpts, &plan.tri_oppDiv,
-                            &plan.tri_oppDiv_fpts})
-        ops.insert(ops.end(), v->begin(), v->end());
+      const std::vector<double> ops = tri_operator_blocks(plan);
       c->dops = dalloc(ops.size() * c->asz);
       if (c->asz == sizeof(double))
         CK(cudaMemcpy(c->dops, ops.data(), ops.size() * sizeof(double), cudaMemcpyHostToDevice));

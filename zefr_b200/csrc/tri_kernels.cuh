@@ -31,17 +31,6 @@ struct TriShape
   static_assert(V == 4, "the shared tile arrays hold four variables per point");
 };
 
-// global [S][V][TW] tile -> the shared layout above
-template <typename T, typename A, int S>
-__device__ __forceinline__ void load_tile_vl(const T *__restrict__ src, A *dst)
-{
-  for (int i = threadIdx.x; i < S * 4 * TW; i += blockDim.x)
-  {
-    const int l = i % TW, v = (i / TW) % 4, p = i / (4 * TW);
-    dst[tix<A>(p, l, v)] = src[i];
-  }
-}
-
 // X_v(f) = sum_s E[f][s] Y_v(s) for the four variables of a shared tile array
 template <typename A, int N>
 __device__ __forceinline__ void tri_extrap4(const A *sY, const A *E, int f, int l, A out[4])
@@ -94,22 +83,6 @@ __global__ void __launch_bounds__(128) k_tri_extrap(const T *__restrict__ U, T *
   }
 }
 
-template <typename T, typename A, int N>
-__device__ __forceinline__ void tri_extrap_next(const Args<T, A> &a, int64_t tile, const A *sUnew, const A *E)
-{
-  using G = TriShape<N>;
-  constexpr int Fp = G::Fp, V = G::V;
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    A x[V];
-    tri_extrap4<A, N>(sUnew, E, f, l, x);
-    T *out = a.Ufp_next + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) out[v * TW] = (T)x[v];
-  }
-}
-
 // transformed flux F~_d = adj[d][.] . F at solution point s into sF [D*S] points
 template <typename A>
 __device__ __forceinline__ void tri_transform(const A F[4][2], const A adj[2][2], A *sF, int S, int s, int l)
@@ -124,244 +97,330 @@ __device__ __forceinline__ void tri_transform(const A F[4][2], const A adj[2][2]
   }
 }
 
-// divF(s) = sum_k oppDiv[s][k] F~(k) + sum_f oppDiv_fpts[s][f] Fc(f), then store / RK
-template <typename T, typename A, int N>
-__device__ __forceinline__ void tri_finish(const Args<T, A> &a, int64_t tile, int s, int l, const A *sF,
-                                           const A *sFc, const A *ops, A *sUnew, const A *vol_in)
+// Launch shape: a thread per solution point and per flux point of a tile, the
+// CTAs resident and walking the tiles, so a kernel's operators are copied to
+// shared memory once per CTA and not once per tile (all five, at P4 14 KB in
+// FP64 beside 4 KB of state per tile; P8 104 KB).  minb: CTAs per SM the
+// registers and the shared memory allow, as resident threads.  Against one
+// 128-thread CTA per tile, us, Navier-Stokes Roe gradient / face with RK
+// update and Euler Rusanov, 2 x 110^2 elements (P6, P8: 2 x 60^2):
+//   FP64  P1 23 -> 15 / 32 -> 18, 30 -> 16;  P3 36 -> 34 / 41 -> 31, 43 -> 32;
+//         P5 112 -> 97 / 86 -> 66, 101 -> 85;  P8 224 -> 111 / 113 -> 51, 142 -> 85
+//   mixed P1 15 -> 13 / 15.5 -> 13, 14 -> 12;  P3 23 -> 23 / 21 -> 20, 22 -> 22;
+//         P5 53 -> 53 / 38 -> 38, 47 -> 45;  P8 82 -> 61 / 46 -> 29, 62 -> 47
+// FP64 face at 512 threads spills the update's inputs: P3 35.
+template <typename A, int N>
+struct TriRun
 {
   using G = TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2;
-  A vol[V], surf[V];
-#pragma unroll
-  for (int v = 0; v < V; v++)
+  static constexpr int items = (G::S > G::Fp ? G::S : G::Fp) * TW;
+  static constexpr int NT = (items + 31) / 32 * 32;
+  static constexpr bool f64 = sizeof(A) == 8;
+  // The operators of a kernel as one block, the two dimensions' rows of oppD,
+  // oppD_fpts and oppDiv interleaved pairwise: element (row, column, d) at
+  // 2 (row * columns + column) + d.  The blocks follow the plain operators in
+  // Args::dops (tri_operator_blocks arranges them).
+  static constexpr int pad(int n) { return (n + 3) / 4 * 4; }
+  static constexpr int GU = 0, GF = GU + 2 * G::S * G::S, GDV = GF + 2 * G::S * G::Fp, GE = GDV + 2 * G::S * G::S,
+                       grad_ops = pad(GE + G::Fp * G::S);
+  static constexpr int FDVF = 0, FE = pad(G::S * G::Fp), face_ops = pad(FE + G::Fp * G::S);
+  static constexpr int EDV = 0, EDVF = 2 * G::S * G::S, EE = pad(EDVF + G::S * G::Fp), euler_ops = pad(EE + G::Fp * G::S);
+  static constexpr int GRAD_AT = pad(G::NOPS), FACE_AT = GRAD_AT + grad_ops, EULER_AT = FACE_AT + face_ops;
+  static constexpr int grad_smem = (grad_ops + (5 * G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
+  static constexpr int face_smem = (face_ops + (G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
+  static constexpr int euler_smem = (euler_ops + (3 * G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
+  static constexpr int fit(int threads, int smem)
   {
-    surf[v] = A(0);
-    vol[v] = A(0);
+    const int by_smem = 225 * 1024 / (smem + 1024), by_threads = threads / NT;
+    const int n = by_smem < by_threads ? by_smem : by_threads;
+    return n < 1 ? 1 : n > 24 ? 24 : n;
   }
-  if (vol_in)
+  static constexpr int grad_minb = fit(f64 ? 512 : 1280, grad_smem);
+  static constexpr int face_minb = fit(f64 ? 400 : 1024, face_smem);
+  static constexpr int euler_minb = fit(f64 ? 512 : 1280, euler_smem);
+};
+
+// a pair of coefficients (dimension 0, dimension 1) with one load
+__device__ __forceinline__ void ld2(const float *p, float &a, float &b)
+{
+  const float2 q = *reinterpret_cast<const float2 *>(p);
+  a = q.x;
+  b = q.y;
+}
+__device__ __forceinline__ void ld2(const double *p, double &a, double &b)
+{
+  const double2 q = *reinterpret_cast<const double2 *>(p);
+  a = q.x;
+  b = q.y;
+}
+
+// copy an operator block (a multiple of 16 bytes, 16-byte aligned) to shared memory
+template <typename A>
+__device__ __forceinline__ void load_block(A *dst, const A *src, int n, int nt)
+{
+  const float4 *g = reinterpret_cast<const float4 *>(src);
+  float4 *d = reinterpret_cast<float4 *>(dst);
+  for (int i = threadIdx.x; i < n * (int)sizeof(A) / 16; i += nt) d[i] = g[i];
+}
+
+// vol = sum_t (oppDiv[s][t] F~_0(t) + oppDiv[s][S + t] F~_1(t)); dv: the row's pairs
+template <typename A, int N>
+__device__ __forceinline__ void tri_divergence(const A *sF, const A *dv, int l, A vol[4])
+{
+  constexpr int S = TriShape<N>::S;
+#pragma unroll
+  for (int v = 0; v < 4; v++) vol[v] = A(0);
+#pragma unroll
+  for (int t = 0; t < S; t++)
   {
+    A c0, c1, x0[4], x1[4];
+    ld2(dv + 2 * t, c0, c1);
+    ld4(sF + tvl<A>(t, l), x0);
+    ld4(sF + tvl<A>(S + t, l), x1);
 #pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = vol_in[v];
+    for (int v = 0; v < 4; v++) vol[v] += c0 * x0[v] + c1 * x1[v];
   }
-  else
-  {
-    const A *Dv = ops + G::ODV + s * D * S;
+}
+
+// surf = sum_f oppDiv_fpts[s][f] Fc(f)
+template <typename A, int N>
+__device__ __forceinline__ void tri_surface(const A *sFc, const A *dvf, int l, A surf[4])
+{
+  constexpr int Fp = TriShape<N>::Fp;
 #pragma unroll
-    for (int k = 0; k < D * S; k++)
-    {
-      A x[4];
-      ld4(sF + tvl<A>(k, l), x);
-#pragma unroll
-      for (int v = 0; v < V; v++) vol[v] += Dv[k] * x[v];
-    }
-  }
-  const A *Dvf = ops + G::ODVF + s * Fp;
+  for (int v = 0; v < 4; v++) surf[v] = A(0);
 #pragma unroll
   for (int f = 0; f < Fp; f++)
   {
     A x[4];
     ld4(sFc + tvl<A>(f, l), x);
 #pragma unroll
-    for (int v = 0; v < V; v++) surf[v] += Dvf[f] * x[v];
+    for (int v = 0; v < 4; v++) surf[v] += dvf[f] * x[v];
   }
-  A res[V], unew[V];
+}
+
+// traces of the updated state (sU, shared) for the next stage
+template <typename T, typename A, int N>
+__device__ __forceinline__ void tri_extrap_next(const Args<T, A> &a, int64_t tile, const A *sU, const A *E, int f,
+                                                int l)
+{
+  A x[4];
+  tri_extrap4<A, N>(sU, E, f, l, x);
+  T *out = a.Ufp_next + (tile * TriShape<N>::Fp + f) * (int64_t)4 * TW + l;
 #pragma unroll
-  for (int v = 0; v < V; v++) res[v] = vol[v] + surf[v];
-  RkIn<A, V> in;
-  if (a.rk_mode) rk_load<T, A, S, V, 5>(a, tile, s, l, in);
-  store_rk<T, A, S, V>(a, tile, s, l, res, in, unew);
-  if (sUnew) st4(sUnew + tvl<A>(s, l), unew);
+  for (int v = 0; v < 4; v++) out[v * TW] = (T)x[v];
 }
 
 // ---------------------------------------------------------------------------
 // Euler: volume flux, common flux and divergence of one tile.
 // ---------------------------------------------------------------------------
 template <typename T, typename A, int N>
-__global__ void __launch_bounds__(128) k_tri_euler(const __grid_constant__ Args<T, A> a)
+__global__ void __launch_bounds__(TriRun<A, N>::NT, TriRun<A, N>::euler_minb)
+    k_tri_euler(const __grid_constant__ Args<T, A> a)
 {
   using G = TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2;
+  using R = TriRun<A, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2, NT = R::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sops = reinterpret_cast<A *>(smem_raw);
-  A *sU = sops + G::OPS_PAD;  // [S] points: the updated state
+  A *sU = sops + R::euler_ops;  // [S] points: the updated state
   A *sF = sU + S * V * TW;
   A *sFc = sF + D * S * V * TW;
-  load_tri_ops<A, N>(sops, a.dops);
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
+  load_block<A>(sops, a.dops + R::EULER_AT, R::euler_ops, NT);
+  const int p = threadIdx.x / TW, l = threadIdx.x % TW;
+  const bool has_s = p < S, has_f = p < Fp;
+  for (int64_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
   {
-    const int s = it / TW, l = it % TW;
-    const T *u = a.U + (tile * S + s) * (int64_t)V * TW + l;
-    const T *m = a.mets + (tile * S + s) * (int64_t)5 * TW + l;
-    A U[V], F[V][D], P, Pp;
+    if (has_s)
+    {
+      const T *u = a.U + (tile * S + p) * (int64_t)V * TW + l;
+      const T *m = a.mets + (tile * S + p) * (int64_t)5 * TW + l;
+      A U[V], F[V][D], P, Pp;
 #pragma unroll
-    for (int v = 0; v < V; v++) U[v] = u[v * TW];
-    const A adj[2][2] = {{m[0], m[TW]}, {m[2 * TW], m[3 * TW]}};
-    flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
-    tri_transform<A>(F, adj, sF, S, s, l);
-  }
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    A out[V];
-    common_flux_2d<T, A, false>(a, tile, Fp, f, l, out);
-    st4(sFc + tvl<A>(f, l), out);
-  }
-  __syncthreads();
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    tri_finish<T, A, N>(a, tile, s, l, sF, sFc, sops, a.extrap_next ? sU : nullptr, nullptr);
-  }
-  if (a.extrap_next)
-  {
+      for (int v = 0; v < V; v++) U[v] = u[v * TW];
+      const A adj[2][2] = {{m[0], m[TW]}, {m[2 * TW], m[3 * TW]}};
+      flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
+      tri_transform<A>(F, adj, sF, S, p, l);
+    }
+    if (has_f)
+    {
+      A out[V];
+      common_flux_2d<T, A, false>(a, tile, Fp, p, l, out);
+      st4(sFc + tvl<A>(p, l), out);
+    }
     __syncthreads();
-    tri_extrap_next<T, A, N>(a, tile, sU, sops + G::OE);
+    if (has_s)
+    {
+      RkIn<A, V> in;
+      if (a.rk_mode) rk_load<T, A, S, V, 5>(a, tile, p, l, in);
+      A res[V], surf[V], unew[V];
+      tri_divergence<A, N>(sF, sops + R::EDV + 2 * p * S, l, res);
+      tri_surface<A, N>(sFc, sops + R::EDVF + p * Fp, l, surf);
+#pragma unroll
+      for (int v = 0; v < V; v++) res[v] += surf[v];
+      store_rk<T, A, S, V>(a, tile, p, l, res, in, unew);
+      if (a.extrap_next) st4(sU + tvl<A>(p, l), unew);
+    }
+    __syncthreads();
+    // the next tile's sU is written only after its own barrier, past this read
+    if (a.extrap_next && has_f) tri_extrap_next<T, A, N>(a, tile, sU, sops + R::EE, p, l);
   }
 }
 
 // ---------------------------------------------------------------------------
 // Navier-Stokes kernel 1: LDG common solution, corrected gradient, own viscous
-// normal flux, volume flux and its divergence.
+// normal flux, volume flux and its divergence.  A point's flux follows its
+// gradient from registers, so the faces need not wait before it.
 // ---------------------------------------------------------------------------
 template <typename T, typename A, int N>
-__global__ void __launch_bounds__(128) k_tri_ns_grad(const __grid_constant__ Args<T, A> a)
+__global__ void __launch_bounds__(TriRun<A, N>::NT, TriRun<A, N>::grad_minb)
+    k_tri_ns_grad(const __grid_constant__ Args<T, A> a)
 {
   using G = TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2, NM = 5;
+  using R = TriRun<A, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2, NM = 5, NT = R::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sops = reinterpret_cast<A *>(smem_raw);
-  A *sU = sops + G::OPS_PAD;    // [S] points
+  A *sU = sops + R::grad_ops;    // [S] points
   A *sUC = sU + S * V * TW;      // [Fp] points
   A *sdU = sUC + Fp * V * TW;    // [D*S] points: physical gradient
   A *sF = sdU + D * S * V * TW;  // [D*S] points: transformed flux
-  load_tri_ops<A, N>(sops, a.dops);
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  load_tile_vl<T, A, S>(a.U + tile * (int64_t)S * V * TW, sU);
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
+  load_block<A>(sops, a.dops + R::GRAD_AT, R::grad_ops, NT);
+  const int p = threadIdx.x / TW, l = threadIdx.x % TW;
+  const bool has_s = p < S, has_f = p < Fp;
+  for (int64_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
   {
-    const int f = it / TW, l = it % TW;
-    const int code = a.nbr[(tile * Fp + f) * (int64_t)TW + l];
-    A Uo[V], UC[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) Uo[v] = uo[v * TW];
-    common_solution_2d<T, A>(a, tile, Fp, f, l, code, Uo, UC);
-    st4(sUC + tvl<A>(f, l), UC);
-  }
-  __syncthreads();
-  // gradient: oppD U + oppD_fpts Ucomm, then physical; the point's flux right
-  // after it, from registers, so the faces need not wait before it
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A tdU[V][D];
-#pragma unroll
-    for (int d = 0; d < D; d++)
+    A U[V], adj[D][D], det = A(1), Uf[V], UC[V];
+    int code = 0;
+    if (has_s)
     {
-      const A *Dd = sops + G::OD + (d * S + s) * S;
-      const A *Df = sops + G::ODF + (d * S + s) * Fp;
-      A acc[V], cor[V];
+      const T *u = a.U + (tile * S + p) * (int64_t)V * TW + l;
+      const T *m = a.mets + (tile * S + p) * (int64_t)NM * TW + l;
 #pragma unroll
-      for (int v = 0; v < V; v++)
-      {
-        acc[v] = A(0);
-        cor[v] = A(0);
-      }
+      for (int v = 0; v < V; v++) U[v] = u[v * TW];
+#pragma unroll
+      for (int d1 = 0; d1 < D; d1++)
+#pragma unroll
+        for (int d2 = 0; d2 < D; d2++) adj[d1][d2] = m[(d1 * D + d2) * TW];
+      det = m[D * D * TW];
+      st4(sU + tvl<A>(p, l), U);
+    }
+    if (has_f)
+    {
+      code = a.nbr[(tile * Fp + p) * (int64_t)TW + l];
+      const T *uo = a.Ufp + (tile * Fp + p) * (int64_t)V * TW + l;
+#pragma unroll
+      for (int v = 0; v < V; v++) Uf[v] = uo[v * TW];
+      common_solution_2d<T, A>(a, tile, Fp, p, l, code, Uf, UC);
+      st4(sUC + tvl<A>(p, l), UC);
+    }
+    __syncthreads();
+    if (has_s)
+    {
+      // oppD U, and apart from it oppD_fpts Ucomm, both dimensions at once
+      A g0[V], g1[V], c0[V], c1[V];
+#pragma unroll
+      for (int v = 0; v < V; v++) g0[v] = g1[v] = c0[v] = c1[v] = A(0);
+      const A *Dd = sops + R::GU + 2 * p * S;
 #pragma unroll
       for (int t = 0; t < S; t++)
       {
-        A x[4];
+        A k0, k1, x[4];
+        ld2(Dd + 2 * t, k0, k1);
         ld4(sU + tvl<A>(t, l), x);
 #pragma unroll
-        for (int v = 0; v < V; v++) acc[v] += Dd[t] * x[v];
+        for (int v = 0; v < V; v++)
+        {
+          g0[v] += k0 * x[v];
+          g1[v] += k1 * x[v];
+        }
       }
+      const A *Df = sops + R::GF + 2 * p * Fp;
 #pragma unroll
       for (int f = 0; f < Fp; f++)
       {
-        A x[4];
+        A k0, k1, x[4];
+        ld2(Df + 2 * f, k0, k1);
         ld4(sUC + tvl<A>(f, l), x);
 #pragma unroll
-        for (int v = 0; v < V; v++) cor[v] += Df[f] * x[v];
+        for (int v = 0; v < V; v++)
+        {
+          c0[v] += k0 * x[v];
+          c1[v] += k1 * x[v];
+        }
       }
-#pragma unroll
-      for (int v = 0; v < V; v++) tdU[v][d] = acc[v] + cor[v];
-    }
-    const T *m = a.mets + (tile * S + s) * (int64_t)NM * TW + l;
-    A adj[D][D];
-#pragma unroll
-    for (int d1 = 0; d1 < D; d1++)
-#pragma unroll
-      for (int d2 = 0; d2 < D; d2++) adj[d1][d2] = m[(d1 * D + d2) * TW];
-    const A inv_det = A(1) / m[D * D * TW];
-    A dU[V][D];
-#pragma unroll
-    for (int d1 = 0; d1 < D; d1++)
-    {
-      A g[V];
 #pragma unroll
       for (int v = 0; v < V; v++)
       {
-        g[v] = (tdU[v][0] * adj[0][d1] + tdU[v][1] * adj[1][d1]) * inv_det;
-        dU[v][d1] = g[v];
+        g0[v] += c0[v];
+        g1[v] += c1[v];
       }
-      st4(sdU + tvl<A>(d1 * S + s, l), g);
-      if (a.dU_out)
+      const A inv_det = A(1) / det;
+      A dU[V][D];
+#pragma unroll
+      for (int d1 = 0; d1 < D; d1++)
       {
-        T *out = a.dU_out + ((tile * D + d1) * S + s) * (int64_t)V * TW + l;
+        A g[V];
 #pragma unroll
-        for (int v = 0; v < V; v++) out[v * TW] = (T)g[v];
+        for (int v = 0; v < V; v++)
+        {
+          g[v] = (g0[v] * adj[0][d1] + g1[v] * adj[1][d1]) * inv_det;
+          dU[v][d1] = g[v];
+        }
+        st4(sdU + tvl<A>(d1 * S + p, l), g);
+        if (a.dU_out)
+        {
+          T *out = a.dU_out + ((tile * D + d1) * S + p) * (int64_t)V * TW + l;
+#pragma unroll
+          for (int v = 0; v < V; v++) out[v * TW] = (T)g[v];
+        }
       }
+      A F[V][D], P, Pp, Ua[V];
+      flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
+      to_abs<A, D>(U, Ua, a.ph);
+      flux_visc_add<A, D>(Ua, dU, F, a.ph);
+      tri_transform<A>(F, adj, sF, S, p, l);
     }
-    A U[V], F[V][D], P, Pp, Ua[V];
-    ld4(sU + tvl<A>(s, l), U);
-    flux_conv_stored<A, D>(U, F, P, Pp, a.ph);
-    to_abs<A, D>(U, Ua, a.ph);
-    flux_visc_add<A, D>(Ua, dU, F, a.ph);
-    tri_transform<A>(F, adj, sF, S, s, l);
-  }
-  __syncthreads();
-  // own viscous normal flux at flux points
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
-  {
-    const int f = it / TW, l = it % TW;
-    const int code = a.nbr[(tile * Fp + f) * (int64_t)TW + l];
-    if (!own_visc_flux(a.ph.ldg_b, code)) continue;
-    A Uf[V], dUf[V][D], UC[V];
-    const T *uo = a.Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) Uf[v] = uo[v * TW];
-    ld4(sUC + tvl<A>(f, l), UC);
-#pragma unroll
-    for (int d = 0; d < D; d++)
+    __syncthreads();
+    // own viscous normal flux at flux points
+    if (has_f && own_visc_flux(a.ph.ldg_b, code))
     {
-      A x[V];
-      tri_extrap4<A, N>(sdU + d * S * V * TW, sops + G::OE, f, l, x);
+      A x0[V], x1[V], dUf[V][D];
 #pragma unroll
-      for (int v = 0; v < V; v++) dUf[v][d] = x[v];
+      for (int v = 0; v < V; v++) x0[v] = x1[v] = A(0);
+      const A *E = sops + R::GE + p * S;
+#pragma unroll
+      for (int t = 0; t < S; t++)
+      {
+        A y0[4], y1[4];
+        ld4(sdU + tvl<A>(t, l), y0);
+        ld4(sdU + tvl<A>(S + t, l), y1);
+        const A e = E[t];
+#pragma unroll
+        for (int v = 0; v < V; v++)
+        {
+          x0[v] += e * y0[v];
+          x1[v] += e * y1[v];
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < V; v++)
+      {
+        dUf[v][0] = x0[v];
+        dUf[v][1] = x1[v];
+      }
+      visc_face_2d<T, A>(a, tile, Fp, p, l, code, Uf, dUf, UC);
     }
-    visc_face_2d<T, A>(a, tile, Fp, f, l, code, Uf, dUf, UC);
-  }
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A vol[V];
-#pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = A(0);
-    const A *Dv = sops + G::ODV + s * D * S;
-#pragma unroll
-    for (int k = 0; k < D * S; k++)
+    if (has_s)
     {
-      A x[V];
-      ld4(sF + tvl<A>(k, l), x);
+      A vol[V];
+      tri_divergence<A, N>(sF, sops + R::GDV + 2 * p * S, l, vol);
+      A *out = a.divF_vol + (tile * S + p) * (int64_t)V * TW + l;
 #pragma unroll
-      for (int v = 0; v < V; v++) vol[v] += Dv[k] * x[v];
+      for (int v = 0; v < V; v++) out[v * TW] = vol[v];
     }
-    A *out = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
-#pragma unroll
-    for (int v = 0; v < V; v++) out[v * TW] = vol[v];
+    // the next tile writes sU and sUC, last read before the barrier above, and
+    // sdU and sF only after its own first barrier
   }
 }
 
@@ -369,38 +428,49 @@ __global__ void __launch_bounds__(128) k_tri_ns_grad(const __grid_constant__ Arg
 // Navier-Stokes kernel 2: convective + LDG common flux, correction, RK.
 // ---------------------------------------------------------------------------
 template <typename T, typename A, int N>
-__global__ void __launch_bounds__(128) k_tri_ns_face(const __grid_constant__ Args<T, A> a)
+__global__ void __launch_bounds__(TriRun<A, N>::NT, TriRun<A, N>::face_minb)
+    k_tri_ns_face(const __grid_constant__ Args<T, A> a)
 {
   using G = TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V;
+  using R = TriRun<A, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V, NT = R::NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   A *sops = reinterpret_cast<A *>(smem_raw);
-  A *sFc = sops + G::OPS_PAD;   // [Fp] points
+  A *sFc = sops + R::face_ops;   // [Fp] points
   A *sUnew = sFc + Fp * V * TW;  // [S] points: the updated state
-  load_tri_ops<A, N>(sops, a.dops);
-  const int64_t tile = blockIdx.x;
-  if (tile >= a.ntiles) return;
-  for (int it = threadIdx.x; it < Fp * TW; it += blockDim.x)
+  load_block<A>(sops, a.dops + R::FACE_AT, a.extrap_next ? R::face_ops : R::FE, NT);
+  const int p = threadIdx.x / TW, l = threadIdx.x % TW;
+  const bool has_s = p < S, has_f = p < Fp;
+  for (int64_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
   {
-    const int f = it / TW, l = it % TW;
-    A out[V];
-    common_flux_2d<T, A, true>(a, tile, Fp, f, l, out);
-    st4(sFc + tvl<A>(f, l), out);
-  }
-  __syncthreads();
-  for (int it = threadIdx.x; it < S * TW; it += blockDim.x)
-  {
-    const int s = it / TW, l = it % TW;
-    A vol[V];
-    const A *dv = a.divF_vol + (tile * S + s) * (int64_t)V * TW + l;
+    RkIn<A, V> in;
+    A res[V];
+    if (has_s)
+    {
+      const A *dv = a.divF_vol + (tile * S + p) * (int64_t)V * TW + l;
 #pragma unroll
-    for (int v = 0; v < V; v++) vol[v] = dv[v * TW];
-    tri_finish<T, A, N>(a, tile, s, l, nullptr, sFc, sops, a.extrap_next ? sUnew : nullptr, vol);
-  }
-  if (a.extrap_next)
-  {
+      for (int v = 0; v < V; v++) res[v] = dv[v * TW];
+      if (a.rk_mode) rk_load<T, A, S, V, 5>(a, tile, p, l, in);
+    }
+    if (has_f)
+    {
+      A out[V];
+      common_flux_2d<T, A, true>(a, tile, Fp, p, l, out);
+      st4(sFc + tvl<A>(p, l), out);
+    }
     __syncthreads();
-    tri_extrap_next<T, A, N>(a, tile, sUnew, sops + G::OE);
+    if (has_s)
+    {
+      A surf[V], unew[V];
+      tri_surface<A, N>(sFc, sops + R::FDVF + p * Fp, l, surf);
+#pragma unroll
+      for (int v = 0; v < V; v++) res[v] += surf[v];
+      store_rk<T, A, S, V>(a, tile, p, l, res, in, unew);
+      if (a.extrap_next) st4(sUnew + tvl<A>(p, l), unew);
+    }
+    __syncthreads();
+    // the next tile's sUnew is written only after its own barrier, past this read
+    if (a.extrap_next && has_f) tri_extrap_next<T, A, N>(a, tile, sUnew, sops + R::FE, p, l);
   }
 }
 

@@ -20,27 +20,24 @@ static void launch_extrap_tri(Ctx &c)
 template <typename T, typename A, int N>
 static void launch_stage_tri(Ctx &c, const StageCfg &sc)
 {
-  using G = dev::TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V, D = 2;
+  using R = dev::TriRun<A, N>;
+  const auto grid = [&](int minb) { return (unsigned)std::min<int64_t>(c.ntiles, (int64_t)148 * minb); };
   const Args<T, A> a = make_args<T, A>(c, sc);
   if (c.tc_err_host && *c.tc_err_host)
   {
     *c.tc_err_host = 0;
     ZB_THROW(ZB_ERR_CUDA, "a tensor-core completion wait of an earlier launch timed out");
   }
-  const size_t ops = (size_t)G::OPS_PAD;
   if (!c.plan.params.viscous)
   {
-    const size_t smem = (ops + (size_t)(S * V + D * S * V + Fp * V) * TW) * sizeof(A);
-    set_smem(dev::k_tri_euler<T, A, N>, smem);
+    set_smem(dev::k_tri_euler<T, A, N>, R::euler_smem);
     ProfScope ps(c, ZB_K_EULER);
-    dev::k_tri_euler<T, A, N><<<(unsigned)c.ntiles, 128, smem, c.stream>>>(a);
+    dev::k_tri_euler<T, A, N><<<grid(R::euler_minb), R::NT, R::euler_smem, c.stream>>>(a);
     c.launches++;
     CK(cudaGetLastError());
   }
   else
   {
-    const size_t smem1 = (ops + (size_t)(S * V + Fp * V + 2 * D * S * V) * TW) * sizeof(A);
     if (!sc.face_only)
     {
       ProfScope ps(c, ZB_K_NS_GRAD);
@@ -58,17 +55,16 @@ static void launch_stage_tri(Ctx &c, const StageCfg &sc)
       }
       if (!launched)
       {
-        set_smem(dev::k_tri_ns_grad<T, A, N>, smem1);
-        dev::k_tri_ns_grad<T, A, N><<<(unsigned)c.ntiles, 128, smem1, c.stream>>>(a);
+        set_smem(dev::k_tri_ns_grad<T, A, N>, R::grad_smem);
+        dev::k_tri_ns_grad<T, A, N><<<grid(R::grad_minb), R::NT, R::grad_smem, c.stream>>>(a);
       }
       c.launches++;
       CK(cudaGetLastError());
     }
     if (sc.grad_only) return;
-    const size_t smem2 = (ops + (size_t)(Fp * V + S * V) * TW) * sizeof(A);
-    set_smem(dev::k_tri_ns_face<T, A, N>, smem2);
+    set_smem(dev::k_tri_ns_face<T, A, N>, R::face_smem);
     ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_tri_ns_face<T, A, N><<<(unsigned)c.ntiles, 128, smem2, c.stream>>>(a);
+    dev::k_tri_ns_face<T, A, N><<<grid(R::face_minb), R::NT, R::face_smem, c.stream>>>(a);
     c.launches++;
     CK(cudaGetLastError());
   }
