@@ -48,8 +48,11 @@ constexpr size_t batch_desc_bytes()
 // [begin, end).  A CTA holds blockDim.x / gsz independent groups of gsz
 // threads (whole warps); each group walks its own share of the items with its
 // own named barrier, so low-order tiles do not leave most of a large CTA idle.
+// Registers held to four CTAs per SM in FP32 (64: the compiler takes 64-79 by
+// itself, the same 445 us per step on 48 cases, n 8-64, P1-P5) and two in FP64
+// (128 against 152-159: 1041 -> 991 us).
 template <typename T, typename A, int NN>
-__global__ void __launch_bounds__(256) k_batch_euler(const BatchCase<T, A> *__restrict__ cases,
+__global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_batch_euler(const BatchCase<T, A> *__restrict__ cases,
                                                      const int2 *__restrict__ items, int begin, int end, int gsz,
                                                      int gstride, int chunk)
 {
