@@ -591,20 +591,26 @@ __global__ void __launch_bounds__(TW * N * N * HexEulerShape<A, N>::zs, HexEuler
 //   face      P2 FP64 33 -> 33 (with the RK update 82 -> 57); mixed stays at
 //             one thread (20 against 25); P4 FP64 44 -> 41 (140 -> 90), mixed
 //             27 -> 25 (61 -> 50)
-// P1 and P3 split their columns in two: in both precisions for the gradient
-// kernel, in FP64 only for the face kernel, which is held to three CTAs per
-// SM (80 registers; some of the RK update's values spill): P3 64^3 0.43
-// against 0.47 ms per residual at two CTAs, 0.57 at four.  P4 with three
-// threads per column spills (96 registers): 262.
+// P1 and P3 split their columns in two.  P1 (40^3): its 64-thread CTAs need
+// more of them per SM than the two or three that suit P3: gradient FP64 141 ->
+// 117 at eight, mixed 64 -> 58 at sixteen; face FP64 43 -> 31 at eight (with
+// the RK update 75 -> 50; LDG beta 0.3 119 -> 77).  P3: the FP64 face kernel is
+// held to three CTAs per SM (80 registers; some of the RK update's values
+// spill): 64^3 0.43 against 0.47 ms per residual at two CTAs, 0.57 at four;
+// the mixed one to four 256-thread CTAs: 24^3 with RK update 40 -> 34, beta 0.3
+// 65 -> 59 (three CTAs 36, one thread per column at eight CTAs 49).  P4 with
+// three threads per column spills (96 registers): gradient 262.
 // ---------------------------------------------------------------------------
 template <typename A, int N>
 struct HexNsShape
 {
   static constexpr bool f64 = sizeof(A) == 8;
   static constexpr int grad_zs = N == 3 ? 3 : 2;
-  static constexpr int grad_minb = N == 3 ? (f64 ? 2 : 4) : N == 5 ? (f64 ? 1 : 2) : (f64 ? 2 : 4);
-  static constexpr int face_zs = f64 ? (N == 3 ? 3 : 2) : (N == 5 ? 2 : 1);
-  static constexpr int face_minb = f64 ? (N == 3 ? 4 : N == 5 ? 2 : 3) : (N == 5 ? 2 : 0);
+  static constexpr int grad_minb =
+      N == 2 ? (f64 ? 8 : 16) : N == 3 ? (f64 ? 2 : 4) : N == 5 ? (f64 ? 1 : 2) : (f64 ? 2 : 4);
+  static constexpr int face_zs = f64 ? (N == 3 ? 3 : 2) : (N >= 4 ? 2 : 1);
+  static constexpr int face_minb =
+      f64 ? (N == 2 ? 8 : N == 3 ? 4 : N == 5 ? 2 : 3) : (N == 5 ? 2 : N == 4 ? 4 : 0);
 };
 
 // ---------------------------------------------------------------------------
