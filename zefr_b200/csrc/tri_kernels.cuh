@@ -55,34 +55,6 @@ __device__ __forceinline__ void load_tri_ops(A *sops, const A *g)
   for (int i = threadIdx.x; i < TriShape<N>::NOPS; i += blockDim.x) sops[i] = g[i];
 }
 
-template <typename T, typename A, int N>
-__global__ void __launch_bounds__(128) k_tri_extrap(const T *__restrict__ U, T *__restrict__ Ufp, int64_t ntiles,
-                                                    const A *__restrict__ dops)
-{
-  using G = TriShape<N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V;
-  __shared__ A sE[Fp * S];
-  for (int i = threadIdx.x; i < Fp * S; i += blockDim.x) sE[i] = dops[G::OE + i];
-  __syncthreads();
-  const int64_t total = ntiles * Fp * TW;
-  for (int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += (int64_t)gridDim.x * blockDim.x)
-  {
-    const int l = (int)(gid % TW);
-    const int f = (int)((gid / TW) % Fp);
-    const int64_t tile = gid / ((int64_t)TW * Fp);
-    const T *Ut = U + tile * (int64_t)S * V * TW;
-    T *out = Ufp + (tile * Fp + f) * (int64_t)V * TW;
-#pragma unroll
-    for (int v = 0; v < V; v++)
-    {
-      A acc = A(0);
-#pragma unroll
-      for (int t = 0; t < S; t++) acc += sE[f * S + t] * (A)Ut[(t * V + v) * TW + l];
-      out[v * TW + l] = (T)acc;
-    }
-  }
-}
-
 // transformed flux F~_d = adj[d][.] . F at solution point s into sF [D*S] points
 template <typename A>
 __device__ __forceinline__ void tri_transform(const A F[4][2], const A adj[2][2], A *sF, int S, int s, int l)
@@ -129,6 +101,7 @@ struct TriRun
   static constexpr int grad_smem = (grad_ops + (5 * G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
   static constexpr int face_smem = (face_ops + (G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
   static constexpr int euler_smem = (euler_ops + (3 * G::S + G::Fp) * 4 * TW) * (int)sizeof(A);
+  static constexpr int extrap_smem = (pad(G::Fp * G::S) + G::S * 4 * TW) * (int)sizeof(A);
   static constexpr int fit(int threads, int smem)
   {
     const int by_smem = 225 * 1024 / (smem + 1024), by_threads = threads / NT;
@@ -138,6 +111,7 @@ struct TriRun
   static constexpr int grad_minb = fit(f64 ? 512 : 1280, grad_smem);
   static constexpr int face_minb = fit(f64 ? 400 : 1024, face_smem);
   static constexpr int euler_minb = fit(f64 ? 512 : 1280, euler_smem);
+  static constexpr int extrap_minb = fit(1536, extrap_smem);
 };
 
 // a pair of coefficients (dimension 0, dimension 1) with one load
@@ -209,6 +183,42 @@ __device__ __forceinline__ void tri_extrap_next(const Args<T, A> &a, int64_t til
   T *out = a.Ufp_next + (tile * TriShape<N>::Fp + f) * (int64_t)4 * TW + l;
 #pragma unroll
   for (int v = 0; v < 4; v++) out[v * TW] = (T)x[v];
+}
+
+// State -> flux points (U_fpts = oppE U_spts).  The tile's state goes through
+// shared memory, so a flux point reads S 16-byte groups there instead of 4 S
+// values through L1: P4 mixed, 24,200 triangles 12.5 -> 10.9 us, FP64 18.8 -> 14.7.
+template <typename T, typename A, int N>
+__global__ void __launch_bounds__(TriRun<A, N>::NT) k_tri_extrap(const T *__restrict__ U, T *__restrict__ Ufp,
+                                                                 int64_t ntiles, const A *__restrict__ dops)
+{
+  using G = TriShape<N>;
+  using R = TriRun<A, N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  A *sE = reinterpret_cast<A *>(smem_raw);
+  A *sU = sE + R::pad(Fp * S);
+  load_block<A>(sE, dops + R::FACE_AT + R::FE, R::pad(Fp * S), R::NT);
+  const int p = threadIdx.x / TW, l = threadIdx.x % TW;
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+  {
+    if (p < S)
+    {
+      const T *u = U + (tile * S + p) * (int64_t)V * TW + l;
+      const A x[V] = {u[0], u[TW], u[2 * TW], u[3 * TW]};
+      st4(sU + tvl<A>(p, l), x);
+    }
+    __syncthreads();
+    if (p < Fp)
+    {
+      A x[V];
+      tri_extrap4<A, N>(sU, sE, p, l, x);
+      T *out = Ufp + (tile * Fp + p) * (int64_t)V * TW + l;
+#pragma unroll
+      for (int v = 0; v < V; v++) out[v * TW] = (T)x[v];
+    }
+    __syncthreads();
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -9,10 +9,12 @@ namespace zb {
 template <typename T, typename A, int N>
 static void launch_extrap_tri(Ctx &c)
 {
-  using G = dev::TriShape<N>;
+  using R = dev::TriRun<A, N>;
+  set_smem(dev::k_tri_extrap<T, A, N>, R::extrap_smem);
   ProfScope ps(c, ZB_K_EXTRAP);
-  dev::k_tri_extrap<T, A, N><<<grid_for(c.ntiles * G::Fp * TW, 128), 128, 0, c.stream>>>(
-      (const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles, (const A *)c.dops);
+  const unsigned grid = (unsigned)std::min<int64_t>(c.ntiles, (int64_t)148 * R::extrap_minb);
+  dev::k_tri_extrap<T, A, N><<<grid, R::NT, R::extrap_smem, c.stream>>>((const T *)c.U, (T *)c.Ufp[c.cur], c.ntiles,
+                                                                        (const A *)c.dops);
   c.launches++;
   CK(cudaGetLastError());
 }
