@@ -131,10 +131,11 @@ static void launch_vjp_tri(Ctx &c, bool params, bool geo)
     return;
   }
   {
-    const size_t smem1 = dev::tri_adj_ns1_smem<N>();
+    using R = dev::TriAdjRun<N>;
+    const size_t smem1 = R::ns1_smem;
     set_smem(dev::k_tri_adj_ns1<N>, smem1);
     ProfScope ps(c, ZB_K_ADJ_VOL);
-    dev::k_tri_adj_ns1<N><<<(unsigned)c.ntiles, 128, smem1, c.stream>>>(a);
+    dev::k_tri_adj_ns1<N><<<(unsigned)c.ntiles, R::ns1_nt, smem1, c.stream>>>(a);
     c.launches++;
     CK(cudaGetLastError());
   }

@@ -22,6 +22,28 @@
 namespace zb {
 namespace dev {
 
+// Launch shape of the Navier-Stokes pass 1.  The pass waits on its own
+// dependent FP64 arithmetic, so it wants every warp the SM can hold: through P4
+// shared memory takes four 128-thread CTAs and the registers are held to them
+// (128; some 800 bytes of the boundary path spilled), at P5 three (168).  From
+// P6 on shared memory takes two CTAs or one, which fit the registers the
+// compiler takes by itself (255), so a bound would only spill (up to 3.2 KB);
+// where it takes one (P7, P8) the CTA has 256 threads.  B200, 2 n^2 elements,
+// us at 238-255 registers and 128 threads / four CTAs at every order / this
+// rule: P3 n 100 Roe 102 / 80 / 80, P4 133 / 123 / 123, P5 225 / 244 / 212,
+// P6 n 80 205 / 315 / 205, P7 505 / 690 / 410, P8 558 / 985 / 442.
+template <int N>
+struct TriAdjRun
+{
+  using G = TriShape<N>;
+  static constexpr size_t ns1_smem =
+      ((size_t)G::OPS_PAD + (size_t)(6 * G::S * 4 + G::Fp * 4) * TW) * sizeof(double);
+  // CTAs per SM by shared memory: 228 KB, per CTA 1 KB reserved and block_sum5's
+  static constexpr int fit = (int)(228 * 1024 / (ns1_smem + 1024 + 32 * 5 * sizeof(double)));
+  static constexpr int minb = fit >= 4 ? 4 : fit == 3 ? 3 : 1;
+  static constexpr int ns1_nt = fit == 1 ? 256 : 128;
+};
+
 // summed weight on the common flux of own flux point f (tensor-product form:
 // face_weight) for the triangle flux-point count
 template <int N>
@@ -202,10 +224,8 @@ __global__ void __launch_bounds__(128) k_tri_adj_euler(const __grid_constant__ A
 // adjoint of the volume flux, of the face fluxes and of the gradient; writes
 // the solution-point part of Ubar, the trace adjoint (Ubfp, and the partner's
 // Riemann part in Ubx) and the common-solution adjoint (UCb)
-// 128 registers, four CTAs per SM (P3 150^2 Roe 230 -> 166 us against 238
-// registers and two; three CTAs 177)
 template <int N>
-__global__ void __launch_bounds__(128, 4) k_tri_adj_ns1(const __grid_constant__ AdjArgs a)
+__global__ void __launch_bounds__(TriAdjRun<N>::ns1_nt, TriAdjRun<N>::minb) k_tri_adj_ns1(const __grid_constant__ AdjArgs a)
 {
   using G = TriShape<N>;
   constexpr int S = G::S, Fp = G::Fp, V = 4, D = 2, NM = 5;
@@ -565,14 +585,6 @@ __global__ void __launch_bounds__(128) k_tri_adj_ns2(const __grid_constant__ Adj
 #pragma unroll
     for (int v = 0; v < V; v++) out[v * TW] = acc[v];
   }
-}
-
-template <int N>
-constexpr size_t tri_adj_ns1_smem()
-{
-  using G = TriShape<N>;
-  return ((size_t)G::OPS_PAD + (size_t)(G::S * 4 + G::Fp * 4 + 2 * G::S * 4 + G::S * 4 + 2 * G::S * 4) * TW) *
-         sizeof(double);
 }
 
 template <int N>
