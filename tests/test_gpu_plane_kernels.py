@@ -70,3 +70,65 @@ def test_many_tiles_repeat_the_few(kind, n):
     assert np.array_equal(R, s.residual(U))
     C = np.broadcast_to(np.array([1.0, 0.3, -0.2, 2.7])[None, :, None], s.state_shape)
     assert np.abs(s.residual(C)).max() < 1e-12
+
+
+# Meshes (box_tris(n): 2 n^2 elements, 8 to a tile) of more tiles than the
+# GPU holds CTAs of any triangle kernel of that order and form (148 SMs times
+# the most CTAs per SM: 20, 13, 13, 3 of the FP32 gradient and Euler kernels at
+# P1, P2, P3, P8, 16, 16, 4 of the extrapolation from P2 on; FP64 8, 5, 5, 1):
+# every CTA walks on to another tile, in FP64 to several.  At P2 this is also
+# where the extrapolation takes its other form.
+MANY = [("fp64", 1, 125), ("fp64", 2, 100), ("mixed", 2, 100), ("fp64", 3, 100), ("fp64", 8, 45), ("mixed", 1, 125), ("mixed", 3, 105), ("mixed", 8, 52)]
+
+
+@pytest.mark.parametrize("viscous,beta,fconv", [(False, 0.5, "roe"), (True, 0.5, "rusanov"), (True, 0.3, "roe")])
+@pytest.mark.parametrize("precision,order,n", MANY)
+def test_triangles_of_more_tiles_than_resident_ctas(precision, order, n, viscous, beta, fconv):
+    """Residual and step against the oracle on a state that differs from tile
+    to tile (random jumps), so a CTA that read what its last tile left behind
+    would show.  Tolerances as in test_residual_and_step; the step adds a
+    multiple of dt / h of the residual's error, both small."""
+    dt = 1e-6
+    s = _case("tri", (n,), order, viscous, beta, fconv, precision, dt)
+    st = O.Setup.from_arrays(2, s.nspts, s.info.nfpts, s.neles, s.plan.get)
+    U, d = _state(s), dict(PHYS, ldg_b=beta)
+    tol = 2e-12 if precision == "fp64" else 1e-4
+    want = O.residual(st, U, d, viscous, fconv)
+    scale = np.abs(want).max(axis=(0, 2))
+    assert (np.abs(s.residual(U) - want).max(axis=(0, 2)) <= tol * scale).all()
+    s.set_state(U)
+    s.step(1)
+    Us, regs = U, [want]
+    for a in (0.5, 0.5, 1.0):
+        Us = U - a * dt / st.jaco_det[:, None] * regs[-1]
+        regs.append(O.residual(st, Us, d, viscous, fconv))
+    Un = U - dt / st.jaco_det[:, None] * (regs[0] + 2 * regs[1] + 2 * regs[2] + regs[3]) / 6
+    moved = np.abs(Un - U).max()
+    err = np.abs(s.get_state() - Un).max()
+    assert err <= (1e-13 + tol * moved if precision == "fp64" else 1e-6)
+    s.close()
+
+
+# every boundary kind through the two-dimensional kernels
+WALLS = [("wall_ns_adi", True), ("wall_ns_iso", True), ("char", True), ("char", False), ("wall_slip", False)]
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 2e-12), ("mixed", 1e-4)])
+@pytest.mark.parametrize("bc,viscous", WALLS)
+@pytest.mark.parametrize("kind,n,order", [("quad", (5, 4), p) for p in (1, 2, 3, 4, 5)] +
+                         [("tri", (4,), p) for p in (1, 2, 3, 4, 5, 6, 7, 8)])
+def test_boundaries(kind, n, order, bc, viscous, precision, tol):
+    """A box whose four sides are one boundary, at every order, against the
+    oracle (tolerances as in test_residual_and_step)."""
+    mesh = (meshgen.jitter_interior(meshgen.box_quads(*n, 0.0, 1.0, 0.0, 1.0, bnd="SIDE"), 0.02, 3) if kind == "quad"
+            else meshgen.box_tris(*n, jitter=0.1, bnd="SIDE"))
+    p = make_params(order, viscous, gamma=1.4, prandtl=0.71, mu=2e-3, ldg_b=0.5, ldg_tau=0.1, precision=precision,
+                    V_fs=(0.3, 0.1, 0.0), rho_fs=1.0, P_fs=1.0, T_wall=1.0, R_ref=1.0)
+    s = FRSolver(mesh, p, {"SIDE": bc})
+    st = O.Setup.from_arrays(2, s.nspts, s.info.nfpts, s.neles, s.plan.get)
+    U = _state(s)
+    d = dict(PHYS, ldg_b=0.5, V_fs0=0.3, V_fs1=0.1, T_wall=1.0, R_ref=1.0)
+    want = O.residual(st, U, d, viscous)
+    scale = np.abs(want).max(axis=(0, 2))
+    assert (np.abs(s.residual(U) - want).max(axis=(0, 2)) <= tol * scale).all()
+    s.close()

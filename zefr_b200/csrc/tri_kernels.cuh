@@ -185,9 +185,48 @@ __device__ __forceinline__ void tri_extrap_next(const Args<T, A> &a, int64_t til
   for (int v = 0; v < 4; v++) out[v * TW] = (T)x[v];
 }
 
-// State -> flux points (U_fpts = oppE U_spts).  The tile's state goes through
-// shared memory, so a flux point reads S 16-byte groups there instead of 4 S
-// values through L1: P4 mixed, 24,200 triangles 12.5 -> 10.9 us, FP64 18.8 -> 14.7.
+// State -> flux points (U_fpts = oppE U_spts), a thread per (flux point, element)
+// reading its S values of every variable through L1.
+template <typename T, typename A, int N>
+__global__ void __launch_bounds__(128) k_tri_extrap_direct(const T *__restrict__ U, T *__restrict__ Ufp, int64_t ntiles,
+                                                           const A *__restrict__ dops)
+{
+  using G = TriShape<N>;
+  constexpr int S = G::S, Fp = G::Fp, V = G::V;
+  __shared__ A sE[Fp * S];
+  for (int i = threadIdx.x; i < Fp * S; i += blockDim.x) sE[i] = dops[G::OE + i];
+  __syncthreads();
+  const int64_t total = ntiles * Fp * TW;
+  for (int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < total; gid += (int64_t)gridDim.x * blockDim.x)
+  {
+    const int l = (int)(gid % TW), f = (int)((gid / TW) % Fp);
+    const int64_t tile = gid / ((int64_t)TW * Fp);
+    const T *u = U + tile * (int64_t)S * V * TW + l;
+    T *out = Ufp + (tile * Fp + f) * (int64_t)V * TW + l;
+#pragma unroll
+    for (int v = 0; v < V; v++)
+    {
+      A acc = A(0);
+#pragma unroll
+      for (int t = 0; t < S; t++) acc += sE[f * S + t] * (A)u[(t * V + v) * TW];
+      out[v * TW] = (T)acc;
+    }
+  }
+}
+
+// The same with the tile's state in shared memory: a flux point reads S 16-byte
+// groups there instead of 4 S values, for two barriers per tile.  us, 2 n^2
+// triangles, direct -> this form, FP64 and mixed: P4 n 110 18.6 -> 14.6 and 12.7
+// -> 10.8, P3 n 110 12.6 -> 10.5 and 10.1 -> 8.7.  At P1 a tile's 48 traces are
+// less work than the barriers (n 110 7.6 -> 8.5 and 6.7 -> 8.3, n 300 14.2 ->
+// 15.8 and 11.5 -> 13.7), and at P2 where CTAs take more than one tile (n 60
+// 8.6 -> 6.8 and 6.9 -> 6.4, n 110 equal, n 300 24.9 -> 26.9 and 17.2 -> 19.4).
+template <int N>
+constexpr bool tri_extrap_direct(int64_t ntiles, int64_t resident_ctas)
+{
+  return N == 2 || (N == 3 && ntiles > resident_ctas);
+}
+
 template <typename T, typename A, int N>
 __global__ void __launch_bounds__(TriRun<A, N>::NT) k_tri_extrap(const T *__restrict__ U, T *__restrict__ Ufp,
                                                                  int64_t ntiles, const A *__restrict__ dops)
