@@ -1,9 +1,11 @@
 // Host-side check of the boundary face reverse (bnd_face_vjp) and its
 // free-stream part against forward-mode dual numbers through the whole face
 // function: common flux with the ghost state, viscous normal flux of the
-// prescribed state and gradient, LDG penalty.  Prints the worst relative error
-// and exits non-zero above 1e-12 (values and weights of order one; a few
-// hundred rounded operations of 1e-16 each).
+// prescribed state and gradient, LDG penalty.  The reverse adds to sums that
+// already hold values, as in the kernels, and the Rusanov dissipation is scaled
+// by 1 - rus_k.  Prints the worst relative error and exits non-zero above 1e-12
+// (values and weights of order one; a few hundred rounded operations of 1e-16
+// each).
 #include <cstdio>
 #include <cstring>
 #include <random>
@@ -36,7 +38,7 @@ static void face(int bc, const DD U[D + 2], const DD dU[D + 2][D], const DD n[D]
 }
 
 template <int D, bool VISC>
-static void check(std::mt19937_64 &rng, int bc, int fconv, bool sutherland, double mach)
+static void check(std::mt19937_64 &rng, int bc, int fconv, bool sutherland, double mach, double rus_k)
 {
   constexpr int V = D + 2;
   std::uniform_real_distribution<double> u(-1.0, 1.0);
@@ -50,6 +52,7 @@ static void check(std::mt19937_64 &rng, int bc, int fconv, bool sutherland, doub
   ph.fix_vis = sutherland ? 0 : 1;
   ph.fconv = fconv;
   ph.ldg_tau = 0.1;
+  ph.rus_k = rus_k;
   ph.rho_fs = 1.1;
   ph.P_fs = 0.9;
   ph.T_wall = 1.2;
@@ -75,7 +78,14 @@ static void check(std::mt19937_64 &rng, int bc, int fconv, bool sutherland, doub
     w[v] = u(rng);
     for (int d = 0; d < D; d++) dU[v][d] = u(rng);
   }
-  double Ub[V] = {0}, dUb[V][D] = {{0}}, pb[5] = {0};
+  // the sums before the call
+  double Ub0[V], dUb0[V][D], pb0[5], Ub[V], dUb[V][D], pb[5];
+  for (int v = 0; v < V; v++)
+  {
+    Ub[v] = Ub0[v] = u(rng);
+    for (int d = 0; d < D; d++) dUb[v][d] = dUb0[v][d] = u(rng);
+  }
+  for (int k = 0; k < 5; k++) pb[k] = pb0[k] = u(rng);
   bnd_face_vjp<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
   const int np = bc_uses_freestream(bc) ? 5 : 0;
   for (int k = 0; k < V + V * D + np; k++)
@@ -94,10 +104,13 @@ static void check(std::mt19937_64 &rng, int bc, int fconv, bool sutherland, doub
     face<D, VISC>(bc, L, dL, nd, q, F);
     double acc = 0.0;
     for (int v = 0; v < V; v++) acc += w[v] * F[v].d;
-    record(bc, kp >= 0 ? pb[kp] : k < V ? Ub[k] : dUb[(k - V) / D][(k - V) % D], acc);
+    const int v = (k - V) / D, d = (k - V) % D;
+    record(bc, kp >= 0 ? pb[kp] : k < V ? Ub[k] : dUb[v][d],
+           (kp >= 0 ? pb0[kp] : k < V ? Ub0[k] : dUb0[v][d]) + acc);
   }
-  if (np == 0)
-    for (int k = 0; k < 5; k++) record(bc, pb[k], 0.0);
+  // parameters that the face does not depend on keep their sums
+  for (int k = 0; k < 5; k++)
+    if (np == 0 || (k >= 1 && k <= 3 && k > D)) record(bc, pb[k], pb0[k]);
 }
 
 int main()
@@ -109,10 +122,11 @@ int main()
       for (int fconv : {0, 2})
       {
         const double mach = rep % 2 ? 0.4 : 2.0;  // sub- and supersonic far fields
-        check<2, true>(rng, bc, fconv, rep % 3 == 0, mach);
-        check<3, true>(rng, bc, fconv, rep % 3 == 1, mach);
-        check<2, false>(rng, bc, fconv, false, mach);
-        check<3, false>(rng, bc, fconv, false, mach);
+        const double rus_k = rep % 4 < 2 ? 0.0 : 0.35;
+        check<2, true>(rng, bc, fconv, rep % 3 == 0, mach, rus_k);
+        check<3, true>(rng, bc, fconv, rep % 3 == 1, mach, rus_k);
+        check<2, false>(rng, bc, fconv, false, mach, rus_k);
+        check<3, false>(rng, bc, fconv, false, mach, rus_k);
       }
   std::printf("worst relative error %.3g\n", g_worst);
   return g_worst <= 1e-12 ? 0 : 1;

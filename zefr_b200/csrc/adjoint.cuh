@@ -652,15 +652,46 @@ ZB_HD_COLD void bnd_face_vjp_cold(int bc, const double U[D + 2], const double dU
 {
   bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
 }
-template <int D, bool VISC>
+// COPY (hexahedra): call the out-of-line form through copies of its arguments.
+// The call takes addresses, and an array whose address is taken lies in local
+// memory on the interior faces as well.  us at 24^3 Rusanov, without -> with:
+// k_adj_euler P1 55.8 -> 49.5, P2 119 -> 105, P3 183 -> 160; k_adj_ns1 P3 404 ->
+// 384 (its geometry form, full of registers as it is, 830 -> 843: not there).
+template <int D, bool VISC, bool COPY = true>
 ZB_HD_INLINE void bnd_face_vjp(int bc, const double U[D + 2], const double dU[D + 2][D], const double n[D],
                                const double w[D + 2], const Phys<double> &ph, double Ub[D + 2],
                                double dUb[D + 2][D], double *pb)
 {
+  constexpr int V = D + 2;
   if constexpr (D == 2)
     bnd_face_vjp_body<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
-  else
+  else if constexpr (!COPY)
     bnd_face_vjp_cold<D, VISC>(bc, U, dU, n, w, ph, Ub, dUb, pb);
+  else
+  {
+    double Uc[V], dUc[V][D], nc[D], wc[V], Ubc[V], dUbc[V][D], pc[5];
+    for (int v = 0; v < V; v++)
+    {
+      Uc[v] = U[v];
+      wc[v] = w[v];
+      Ubc[v] = Ub[v];
+      for (int d = 0; d < D; d++)
+      {
+        dUc[v][d] = dU[v][d];
+        dUbc[v][d] = dUb[v][d];
+      }
+    }
+    for (int d = 0; d < D; d++) nc[d] = n[d];
+    for (int k = 0; k < 5; k++) pc[k] = pb ? pb[k] : 0.0;
+    bnd_face_vjp_cold<D, VISC>(bc, Uc, dUc, nc, wc, ph, Ubc, dUbc, pb ? pc : nullptr);
+    for (int v = 0; v < V; v++)
+    {
+      Ub[v] = Ubc[v];
+      for (int d = 0; d < D; d++) dUb[v][d] = dUbc[v][d];
+    }
+    if (pb)
+      for (int k = 0; k < 5; k++) pb[k] = pc[k];
+  }
 }
 
 // Ub += (d UB / d U)^T w for the prescribed boundary state UB of the LDG
@@ -1527,7 +1558,7 @@ __global__ void __launch_bounds__(Shape<D, N>::NT, adj_ns1_minb<D, N, GEO>()) k_
     }
     else
     {
-      bnd_face_vjp<D, true>(-code - 1, Uo, dUo, n, w, a.ph, Ub, dUb, a.pbar ? pb : nullptr);
+      bnd_face_vjp<D, true, !GEO>(-code - 1, Uo, dUo, n, w, a.ph, Ub, dUb, a.pbar ? pb : nullptr);
     }
     if (GEO && a.gbar) geo_face_ns<D, N>(a, tile, f, l, code, n, w, Uo, dUo);
     double *ub = a.Ubfp + (tile * Fp + f) * (int64_t)V * TW + l;
