@@ -44,7 +44,7 @@ static void quad()
 {
   using O = QuadOcc<A, N>;
   held("quad gradient", N, sizeof(A), O::grad, quad_grad_smem_elems<N>() * sizeof(A), QuadShape<N>::NT);
-  held("quad face", N, sizeof(A), O::face, quad_face_smem_elems<N>() * sizeof(A), QuadShape<N>::NT);
+  held("quad face", N, sizeof(A), O::face_many, quad_face_smem_elems<N>() * sizeof(A), QuadShape<N>::NT);
   held("quad Euler", N, sizeof(A), O::euler, euler_smem_elems<N>() * sizeof(A), QuadShape<N>::NT);
 }
 

@@ -60,6 +60,14 @@ def test_residual_and_step(kind, n, order, viscous, beta, fconv, precision, tol)
     assert np.abs(s.get_state() - Un).max() <= (1e-13 if precision == "fp64" else 1e-6)
 
 
+@pytest.mark.parametrize("precision,tol", [("fp64", 2e-12), ("mixed", 1e-4)])
+@pytest.mark.parametrize("beta,fconv", [(0.5, "roe"), (0.3, "rusanov")])
+def test_quads_p5_of_more_tiles_than_sms(beta, fconv, precision, tol):
+    """154 tiles: the FP64 face kernel takes its two-CTA form past 148
+    (tolerances as in test_residual_and_step)."""
+    test_residual_and_step("quad", (41, 30), 5, True, beta, fconv, precision, tol)
+
+
 @pytest.mark.parametrize("kind,n", [("quad", (123, 97)), ("tri", (91,))])
 def test_many_tiles_repeat_the_few(kind, n):
     """More tiles than fit the GPU at once: a uniform state stays uniform and

@@ -279,8 +279,10 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
       dev::k_ns_grad<double, double, N><<<(unsigned)p.ntiles, NT, smem1, st>>>(a, ops);
       NA_CK(cudaGetLastError());
       const size_t smem2 = dev::quad_face_smem_elems<N>() * sizeof(double);
-      NA_CK(cudaFuncSetAttribute(dev::k_ns_face<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
-      dev::k_ns_face<double, double, N><<<(unsigned)p.ntiles, NT, smem2, st>>>(a, ops);
+      using O = dev::QuadOcc<double, N>;
+      auto face = p.ntiles > 148 ? dev::k_ns_face<double, double, N, O::face_many> : dev::k_ns_face<double, double, N, O::face>;
+      NA_CK(cudaFuncSetAttribute(face, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+      face<<<(unsigned)p.ntiles, NT, smem2, st>>>(a, ops);
       NA_CK(cudaGetLastError());
     }
   }

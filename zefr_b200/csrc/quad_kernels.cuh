@@ -31,7 +31,12 @@ struct QuadShape
 // per tile).  FP32 P4, 140^2 elements, us at 1024 / 1280 / 1536 threads:
 // gradient 24.2 / 23.1 / 24.3, Euler 25.2 / 23.5 / 23.8, face with RK update
 // 23.7 / 23.7 / 25.9 (P2: 14.2 / 15.3 / 17.0).  FP64 at 512, 640 and 768 is
-// within 1% of itself; 512 spills least.
+// within 1% of itself; 512 spills least.  512 threads are one CTA of P5's 288,
+// too few for the FP64 face kernel where an SM has more than one tile to do:
+// `face_many` CTAs then (P5: two of 96 registers, some spilled).  P5 FP64 face,
+// n^2 elements, LDG beta 0.3 Rusanov, us at one -> two: n 60 14.2 -> 12.5 (with
+// the RK update 17.3 -> 15.1), n 140 51.5 -> 43.4 (73.3 -> 59.5); beta 0.5 Roe
+// n 140 51.6 -> 50.9 (75.2 -> 68.3); n 24, fewer tiles than SMs, 8.9 -> 10.1.
 template <typename A, int N>
 struct QuadOcc
 {
@@ -39,6 +44,7 @@ struct QuadOcc
   static constexpr bool f64 = sizeof(A) == 8;
   static constexpr int grad = (f64 ? 512 : 1280) / nt, face = (f64 ? 512 : 1024) / nt,
                        euler = (f64 ? 512 : 1280) / nt;
+  static constexpr int face_many = face > 1 ? face : 2;
 };
 
 // X_v(f) of the four variables of a shared tile array at flux point f
@@ -385,8 +391,8 @@ constexpr int quad_face_smem_elems()
 // The point's volume residual and update inputs load while the face flux is
 // formed.
 // ---------------------------------------------------------------------------
-template <typename T, typename A, int N>
-__global__ void __launch_bounds__(QuadShape<N>::NT, QuadOcc<A, N>::face)
+template <typename T, typename A, int N, int MINB>
+__global__ void __launch_bounds__(QuadShape<N>::NT, MINB)
     k_ns_face(const __grid_constant__ Args<T, A> a, const __grid_constant__ LineOpsT<A, N> ops)
 {
   using G = QuadShape<N>;

@@ -16,6 +16,17 @@ static void launch_extrap_quad(Ctx &c)
   CK(cudaGetLastError());
 }
 
+template <typename T, typename A, int N, int MINB>
+static void launch_face_quad(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
+{
+  const size_t smem = dev::quad_face_smem_elems<N>() * sizeof(A);
+  set_smem(dev::k_ns_face<T, A, N, MINB>, smem);
+  ProfScope ps(c, ZB_K_NS_FACE);
+  dev::k_ns_face<T, A, N, MINB><<<(unsigned)c.ntiles, dev::QuadShape<N>::NT, smem, c.stream>>>(a, ops);
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
 template <typename T, typename A, int N>
 static void launch_stage_quad(Ctx &c, const StageCfg &sc)
 {
@@ -43,12 +54,11 @@ static void launch_stage_quad(Ctx &c, const StageCfg &sc)
       CK(cudaGetLastError());
     }
     if (sc.grad_only) return;
-    const size_t smem2 = dev::quad_face_smem_elems<N>() * sizeof(A);
-    set_smem(dev::k_ns_face<T, A, N>, smem2);
-    ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_ns_face<T, A, N><<<(unsigned)c.ntiles, NT, smem2, c.stream>>>(a, ops);
-    c.launches++;
-    CK(cudaGetLastError());
+    using O = dev::QuadOcc<A, N>;
+    if (c.ntiles > 148)
+      launch_face_quad<T, A, N, O::face_many>(c, a, ops);
+    else
+      launch_face_quad<T, A, N, O::face>(c, a, ops);
   }
   if (sc.extrap_next) c.cur ^= 1;
 }
