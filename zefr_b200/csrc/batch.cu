@@ -21,7 +21,6 @@ namespace zb {
 
 using dev::Args;
 using dev::LineOpsT;
-using dev::Shape;
 using dev::TW;
 
 constexpr int kBatchMaxN = 6;
@@ -90,14 +89,14 @@ __global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_batch_euler(con
 
 // The single-launch form: one persistent kernel per stage walks the items of
 // every order (costliest order first) and runs each with its order's tile
-// body; the group's shared memory fits the largest order present.  In FP32
-// the registers are held to four 256-thread CTAs per SM: the kernel carries
-// every order's body, and left to itself the compiler sizes it for the
-// largest (128 registers, two CTAs per SM: 38 GDOF/s on the 512-case batch
-// against 44 at four CTAs per SM, a few bytes of the largest order's
-// values spilled).
+// body; the group's shared memory fits the largest order present.  The kernel
+// carries every order's body, and left to itself the compiler sizes it for the
+// largest.  Registers held to four 256-thread CTAs per SM in FP32 (64, 444
+// bytes spilled; three, 80 registers and 348 bytes, 646 -> 680 us per step of
+// 96 cases, n 8-64, P1-P5) and to two in FP64 (128, 1,100 bytes spilled; one,
+// 255 registers and 256 bytes, 1144 -> 1407 us).
 template <typename T, typename A>
-__global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 1) k_batch_euler_fused(const BatchCase<T, A> *__restrict__ cases,
+__global__ void __launch_bounds__(256, sizeof(A) == 4 ? 4 : 2) k_batch_euler_fused(const BatchCase<T, A> *__restrict__ cases,
                                                            const int2 *__restrict__ items, int begin, int end, int gsz,
                                                            int gstride, int chunk)
 {
