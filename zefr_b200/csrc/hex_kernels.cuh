@@ -581,25 +581,17 @@ __global__ void __launch_bounds__(TW * N * N * HexEulerShape<A, N>::zs, HexEuler
 }
 
 // ---------------------------------------------------------------------------
-// Launch shape of the Navier-Stokes kernels.  zs threads share each (element,
+// Launch shape of the gradient kernel.  zs threads share each (element,
 // x, y) column (z-levels and flux points dealt out between them), multiplying
 // the warps per CTA for the same shared memory; minb is the CTAs per SM the
 // register allocation is held to (0: the compiler's choice).  Timed on B200,
 // us per residual on jittered boxes (P2 29^3, P4 20^3), zs = 1 -> this table:
 //   gradient  P2 FP64 219 -> 145, mixed 115 -> 82; P4 FP64 227 -> 217 (LDG
 //             beta 0.3: 246 -> 220), mixed 133 -> 118 (127 -> 109)
-//   face      P2 FP64 33 -> 33 (with the RK update 82 -> 57); mixed stays at
-//             one thread (20 against 25); P4 FP64 44 -> 41 (140 -> 90), mixed
-//             27 -> 25 (61 -> 50)
 // P1 and P3 split their columns in two.  P1 (40^3): its 64-thread CTAs need
-// more of them per SM than the two or three that suit P3: gradient FP64 141 ->
-// 117 at eight, mixed 64 -> 58 at sixteen; face FP64 43 -> 31 at eight (with
-// the RK update 75 -> 50; LDG beta 0.3 119 -> 77).  P3: the FP64 face kernel is
-// held to three CTAs per SM (80 registers; some of the RK update's values
-// spill): 64^3 0.43 against 0.47 ms per residual at two CTAs, 0.57 at four;
-// the mixed one to four 256-thread CTAs: 24^3 with RK update 40 -> 34, beta 0.3
-// 65 -> 59 (three CTAs 36, one thread per column at eight CTAs 49).  P4 with
-// three threads per column spills (96 registers): gradient 262.
+// more of them per SM than the two or three that suit P3: FP64 141 -> 117 at
+// eight, mixed 64 -> 58 at sixteen.  P4 with three threads per column spills (96
+// registers): 262.
 // ---------------------------------------------------------------------------
 template <typename A, int N>
 struct HexNsShape
@@ -608,9 +600,35 @@ struct HexNsShape
   static constexpr int grad_zs = N == 3 ? 3 : 2;
   static constexpr int grad_minb =
       N == 2 ? (f64 ? 8 : 16) : N == 3 ? (f64 ? 2 : 4) : N == 5 ? (f64 ? 1 : 2) : (f64 ? 2 : 4);
-  static constexpr int face_zs = f64 ? (N == 3 ? 3 : 2) : (N >= 4 ? 2 : 1);
-  static constexpr int face_minb =
-      f64 ? (N == 2 ? 8 : N == 3 ? 4 : N == 5 ? 2 : 3) : (N == 5 ? 2 : N == 4 ? 4 : 0);
+};
+
+// Launch shape of the face kernel, by what it does.  ONE: the one-sided form,
+// which gathers the common flux that the gradient kernel formed, against the
+// trace-buffer form, which solves the Riemann problems itself (twice the
+// registers); RK: with the update (its inputs live across the surface sum)
+// against a residual alone.  FP64 splits every column, the Riemann form with
+// fewer CTAs per SM so that little spills (P2 two of 128 registers: four of 72
+// spilled 580 bytes); the mixed form splits but for the one-sided residual of
+// P3 and P4.  B200, Roe, jittered boxes, us: one shape for all four / this:
+//   one-sided residual   FP64 P1 44^3 39 / 32, P2 30^3 32 / 31, P3 48^3 187 /
+//                        158, P4 20^3 41 / 31; mixed 22.8 / 22.4, 22.8 / 20.8,
+//                        116 / 99, 26 / 21
+//   with the update      FP64 63 / 52, 56 / 53, 384 / 385, 91 / 86; mixed 35 /
+//                        30, 39 / 33, 208 / 202, 48 / 45
+//   trace-buffer residual (beta 0.3)  FP64 99 / 97, 131 / 96, 679 / 509, 115 /
+//                        85; mixed 54 / 49, 53 / 45, 248 / 240, 47 / 45
+//   with the update      FP64 134 / 132, 174 / 159, 983 / 866, 184 / 162; mixed
+//                        68 / 61, 73 / 62, 396 / 394, 74 / 74
+template <typename A, int N, bool ONE, bool RK>
+struct HexFaceShape
+{
+  static constexpr bool f64 = sizeof(A) == 8;
+  static constexpr bool whole = !f64 && ONE && !RK && N >= 4;  // one thread per column
+  static constexpr int zs = whole ? 1 : N == 3 ? 3 : 2;
+  static constexpr int minb = f64   ? (ONE ? (N == 2 ? 12 : N == 3 ? 4 : N == 4 ? (RK ? 3 : 4) : (RK ? 2 : 0))
+                                           : (N == 2 ? 8 : N == 5 ? 1 : 2))
+                              : whole ? (N == 4 ? 6 : 4)
+                                      : (N == 2 ? 20 : N == 3 ? (ONE ? 0 : 5) : N == 4 ? 4 : 2);
 };
 
 // ---------------------------------------------------------------------------
@@ -1045,12 +1063,12 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
 // Navier-Stokes kernel 2 (column mapping): common flux, surface correction,
 // RK update, next-stage extrapolation
 // ---------------------------------------------------------------------------
-template <typename T, typename A, int N>
-__global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsShape<A, N>::face_minb)
+template <typename T, typename A, int N, bool ONE, bool RK>
+__global__ void __launch_bounds__(TW * N * N * HexFaceShape<A, N, ONE, RK>::zs, HexFaceShape<A, N, ONE, RK>::minb)
     k_hex_ns_face(const __grid_constant__ Args<T, A> a, const __grid_constant__ LineOpsT<A, N> ops)
 {
   using H = HexIdx<N>;
-  constexpr int ZS = HexNsShape<A, N>::face_zs;
+  constexpr int ZS = HexFaceShape<A, N, ONE, RK>::zs;
   using Z = ZSplit<N, ZS>;
   constexpr int S = H::S, Fp = H::Fp, V = 5, NZ = Z::NZ;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1064,7 +1082,7 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsS
   o.load(ops, ix, iy);
   int f[6];
   H::fpts(ix, iy, f);
-  if (a.Fcom)
+  if constexpr (ONE)
     hex_gather_common<T, A, N, ZS>(a, tile, l, ix, iy, sFc, zs);
   else
     hex_common_flux<T, A, N, true, ZS>(a, tile, l, ix, iy, sFc, zs);
@@ -1090,9 +1108,15 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::face_zs, HexNsS
     A res[V];
 #pragma unroll
     for (int v = 0; v < V; v++) res[v] = dvol[k][v] + hex_surface<A, N>(ops, o, sFc, ix, iy, iz, v, l);
-    hex_finish<T, A, N>(a, tile, s, l, res, a.extrap_next ? sUnew : nullptr);
+    if constexpr (RK)
+      hex_finish<T, A, N>(a, tile, s, l, res, !ONE && a.extrap_next ? sUnew : nullptr);
+    else
+    {
+#pragma unroll
+      for (int v = 0; v < V; v++) a.divF[(tile * S + s) * (int64_t)V * TW + v * TW + l] = res[v];
+    }
   }
-  if (a.extrap_next)
+  if (RK && !ONE && a.extrap_next)
   {
     __syncthreads();
     hex_extrap_next<T, A, N, ZS>(a, tile, l, ix, iy, f, sUnew, ops, zs);

@@ -6,6 +6,19 @@
 
 namespace zb {
 
+template <typename T, typename A, int N, bool ONE, bool RK>
+static void launch_face_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
+{
+  using G = Shape<3, N>;
+  const size_t smem = (size_t)(G::Fp * G::V + (RK && !ONE ? G::S * G::V : 0)) * TW * sizeof(A);
+  set_smem(dev::k_hex_ns_face<T, A, N, ONE, RK>, smem);
+  ProfScope ps(c, ZB_K_NS_FACE);
+  dev::k_hex_ns_face<T, A, N, ONE, RK>
+      <<<(unsigned)c.ntiles, TW * N * N * dev::HexFaceShape<A, N, ONE, RK>::zs, smem, c.stream>>>(a, ops);
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
 template <typename T, typename A, int N>
 static void launch_extrap_hex(Ctx &c)
 {
@@ -36,7 +49,7 @@ static void launch_stage_hex(Ctx &c, const StageCfg &sc)
   }
   else
   {
-    constexpr int ZG = dev::HexNsShape<A, N>::grad_zs, ZF = dev::HexNsShape<A, N>::face_zs;
+    constexpr int ZG = dev::HexNsShape<A, N>::grad_zs;
     const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(A);  // + sX padding
     set_smem(dev::k_hex_ns_grad<T, A, N>, smem1);
     if (!sc.face_only)
@@ -47,12 +60,10 @@ static void launch_stage_hex(Ctx &c, const StageCfg &sc)
       CK(cudaGetLastError());
     }
     if (sc.grad_only) return;
-    const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(A);
-    set_smem(dev::k_hex_ns_face<T, A, N>, smem2);
-    ProfScope ps(c, ZB_K_NS_FACE);
-    dev::k_hex_ns_face<T, A, N><<<(unsigned)c.ntiles, HT * ZF, smem2, c.stream>>>(a, ops);
-    c.launches++;
-    CK(cudaGetLastError());
+    if (a.Fcom)
+      a.rk_mode ? launch_face_hex<T, A, N, true, true>(c, a, ops) : launch_face_hex<T, A, N, true, false>(c, a, ops);
+    else
+      a.rk_mode ? launch_face_hex<T, A, N, false, true>(c, a, ops) : launch_face_hex<T, A, N, false, false>(c, a, ops);
   }
   if (sc.extrap_next)
   {

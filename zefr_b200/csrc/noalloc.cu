@@ -246,17 +246,22 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
     }
     else
     {
-      constexpr int ZG = dev::HexNsShape<double, N>::grad_zs, ZF = dev::HexNsShape<double, N>::face_zs;
+      constexpr int ZG = dev::HexNsShape<double, N>::grad_zs;
       const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(double);
       NA_CK(cudaFuncSetAttribute(dev::k_hex_ns_grad<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem1));
       dev::k_hex_ns_grad<double, double, N><<<(unsigned)p.ntiles, HT * ZG, smem1, st>>>(a, ops);
       NA_CK(cudaGetLastError());
-      const size_t smem2 = (size_t)(Fp * V + S * V) * TW * sizeof(double);
-      NA_CK(cudaFuncSetAttribute(dev::k_hex_ns_face<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem2));
-      dev::k_hex_ns_face<double, double, N><<<(unsigned)p.ntiles, HT * ZF, smem2, st>>>(a, ops);
-      NA_CK(cudaGetLastError());
+      const size_t smem2 = (size_t)Fp * V * TW * sizeof(double);
+      const auto face = [&](auto kernel, int zs) {
+        NA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2));
+        kernel<<<(unsigned)p.ntiles, HT * zs, smem2, st>>>(a, ops);
+        NA_CK(cudaGetLastError());
+      };
+      if (a.Fcom)
+        face(dev::k_hex_ns_face<double, double, N, true, false>, dev::HexFaceShape<double, N, true, false>::zs);
+      else
+        face(dev::k_hex_ns_face<double, double, N, false, false>, dev::HexFaceShape<double, N, false, false>::zs);
     }
   }
   else
