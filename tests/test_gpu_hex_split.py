@@ -49,3 +49,12 @@ def test_residual_and_step(n, order, viscous, beta, fconv, precision, tol):
     Un = U - 1e-3 / st.jaco_det[:, None] * (regs[0] + 2 * regs[1] + 2 * regs[2] + regs[3]) / 6
     step_tol = 1e-13 if precision == "fp64" else 1e-6
     assert np.abs(s.get_state() - Un).max() <= step_tol
+
+
+@pytest.mark.parametrize("n,order,viscous,beta", [((18, 17, 17), 1, True, 0.5), ((18, 17, 17), 1, True, 0.3),
+                                                  ((16, 16, 16), 2, False, 0.5)])
+def test_shapes_chosen_by_mesh_size(n, order, viscous, beta):
+    """FP64 P1 gradient kernel past the 592 tiles that four CTAs per SM hold (the
+    meshes above stay below), P2 Euler kernel between three and four CTAs per SM
+    (512 tiles); tolerances as above."""
+    test_residual_and_step(n, order, viscous, beta, "rusanov", "fp64", 1e-12)

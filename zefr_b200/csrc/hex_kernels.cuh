@@ -495,11 +495,16 @@ __device__ __forceinline__ void load_adj(const Args<T, A> &a, int64_t tile, int 
 // Launch shape of the Euler kernel: zs threads share a column, minb CTAs per
 // SM bound the registers.  One thread per column left 2-7 warps per CTA beside
 // 18-208 KB (FP64) of shared memory, too few to cover the metric and trace
-// loads; the split costs nothing but the barrier.  Timed on B200 (Rusanov,
-// jittered boxes, us per residual, zs = 1 -> this table): FP64 P1 40^3 77 ->
-// 66, P2 29^3 109 -> 88, P3 24^3 119 -> 87, P4 20^3 150 -> 117; mixed 44 ->
-// 41, 51 -> 43, 56 -> 47, 72 -> 60.  P2 with two threads per column or with
-// four CTAs per SM (72 registers, 400 bytes spilled) was no better than one.
+// loads.  B200, Rusanov, jittered boxes, us per residual, one thread per column
+// -> this table: FP64 P2 29^3 96 -> 78; mixed P1 44^3 50 -> 41, P2 30^3 47 -> 38,
+// P3 36^3 150 -> 125, P4 20^3 68 -> 56.
+//
+// few: the shape where it saves a wave of CTAs.  P2 FP64 holds three of its
+// 216-thread CTAs (80 registers), so a mesh of 445 to 592 tiles took two waves
+// where two threads per column at four CTAs (96 registers) take one; a wave of
+// the latter takes 1.4 times as long (10.5 and 14.8 us).  16^3 (512 tiles) 20.9
+// -> 16.8 us, with the RK update 27.5 -> 21.6; 20^3 31.4 -> 29.7; 29^3, seven
+// waves against six, would be 78 -> 88.
 template <typename A, int N>
 struct HexEulerShape
 {
@@ -509,14 +514,19 @@ struct HexEulerShape
                               : N == 3 ? (f64 ? 3 : 5)
                               : N == 4 ? (f64 ? 2 : 4)
                                        : (f64 ? 1 : 2);
+  static constexpr int few_zs = N == 3 && f64 ? 2 : zs, few_minb = N == 3 && f64 ? 4 : minb;
+  static bool few(int64_t ntiles)
+  {
+    const auto waves = [&](int ctas) { return (ntiles + 148 * ctas - 1) / (148 * ctas); };
+    return few_minb != minb && 7 * waves(few_minb) < 5 * waves(minb);
+  }
 };
 
-template <typename T, typename A, int N>
-__global__ void __launch_bounds__(TW * N * N * HexEulerShape<A, N>::zs, HexEulerShape<A, N>::minb)
+template <typename T, typename A, int N, int ZS, int MINB>
+__global__ void __launch_bounds__(TW * N * N * ZS, MINB)
     k_hex_euler(const __grid_constant__ Args<T, A> a, const __grid_constant__ LineOpsT<A, N> ops)
 {
   using H = HexIdx<N>;
-  constexpr int ZS = HexEulerShape<A, N>::zs;
   using Z = ZSplit<N, ZS>;
   constexpr int S = H::S, V = 5, NZ = Z::NZ;
   extern __shared__ __align__(16) unsigned char smem_raw[];

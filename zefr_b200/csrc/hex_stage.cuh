@@ -6,6 +6,20 @@
 
 namespace zb {
 
+// column-mapped kernels: TW x N^2 threads per tile, times the threads that share
+// a column
+template <typename T, typename A, int N, int ZS, int MINB>
+static void launch_euler_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
+{
+  using G = Shape<3, N>;
+  const size_t smem = (size_t)(4 * G::S * G::V + G::Fp * G::V) * TW * sizeof(A);
+  set_smem(dev::k_hex_euler<T, A, N, ZS, MINB>, smem);
+  ProfScope ps(c, ZB_K_EULER);
+  dev::k_hex_euler<T, A, N, ZS, MINB><<<(unsigned)c.ntiles, TW * N * N * ZS, smem, c.stream>>>(a, ops);
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
 template <typename T, typename A, int N, bool ONE, bool RK>
 static void launch_face_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
 {
@@ -40,12 +54,11 @@ static void launch_stage_hex(Ctx &c, const StageCfg &sc)
   constexpr int HT = TW * N * N;
   if (!c.plan.params.viscous)
   {
-    const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(A);
-    set_smem(dev::k_hex_euler<T, A, N>, smem);
-    ProfScope ps(c, ZB_K_EULER);
-    dev::k_hex_euler<T, A, N><<<(unsigned)c.ntiles, HT * dev::HexEulerShape<A, N>::zs, smem, c.stream>>>(a, ops);
-    c.launches++;
-    CK(cudaGetLastError());
+    using E = dev::HexEulerShape<A, N>;
+    if (E::few(c.ntiles))
+      launch_euler_hex<T, A, N, E::few_zs, E::few_minb>(c, a, ops);
+    else
+      launch_euler_hex<T, A, N, E::zs, E::minb>(c, a, ops);
   }
   else
   {

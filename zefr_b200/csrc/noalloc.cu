@@ -239,10 +239,16 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
     if (!p.params.viscous)
     {
       const size_t smem = (size_t)(S * V + 3 * S * V + Fp * V) * TW * sizeof(double);
-      NA_CK(cudaFuncSetAttribute(dev::k_hex_euler<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-      dev::k_hex_euler<double, double, N><<<(unsigned)p.ntiles, HT * dev::HexEulerShape<double, N>::zs, smem, st>>>(a, ops);
-      NA_CK(cudaGetLastError());
+      using E = dev::HexEulerShape<double, N>;
+      const auto euler = [&](auto kernel, int zs) {
+        NA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<(unsigned)p.ntiles, HT * zs, smem, st>>>(a, ops);
+        NA_CK(cudaGetLastError());
+      };
+      if (E::few(p.ntiles))
+        euler(dev::k_hex_euler<double, double, N, E::few_zs, E::few_minb>, E::few_zs);
+      else
+        euler(dev::k_hex_euler<double, double, N, E::zs, E::minb>, E::zs);
     }
     else
     {
