@@ -591,18 +591,18 @@ __global__ void __launch_bounds__(TW * N * N * ZS, MINB)
 }
 
 // ---------------------------------------------------------------------------
-// Launch shape of the gradient kernel.  zs threads share each (element,
-// x, y) column (z-levels and flux points dealt out between them), multiplying
-// the warps per CTA for the same shared memory; minb is the CTAs per SM the
-// register allocation is held to (0: the compiler's choice).  Timed on B200,
-// us per residual on jittered boxes (P2 29^3, P4 20^3), zs = 1 -> this table:
-//   gradient  P2 FP64 219 -> 145, mixed 115 -> 82; P4 FP64 227 -> 217 (LDG
-//             beta 0.3: 246 -> 220), mixed 133 -> 118 (127 -> 109)
-// P1 and P3 split their columns in two.  P1 (40^3): its 64-thread CTAs need
-// more of them per SM than the two or three that suit P3: FP64 141 -> 117 at
-// eight, mixed 64 -> 58 at sixteen.  P4 with three threads per column spills (96
-// registers): 262.
-// ---------------------------------------------------------------------------
+// Launch shape of the gradient kernel.  zs threads share each (element, x, y)
+// column (z-levels and flux points dealt out between them), multiplying the
+// warps per CTA for the same shared memory; grad_minb is the CTAs per SM the
+// register allocation is held to.  B200, us per residual on jittered boxes, one
+// thread per column at the compiler's registers -> this table: FP64 P1 44^3
+// 162 -> 150, P2 30^3 168 -> 147, P3 40^3 688 -> 548, P4 20^3 228 -> 215; mixed
+// 83 -> 74, 110 -> 80, 371 -> 302, 125 -> 112.  The split at the compiler's
+// registers: FP64 184, 206, 709, 220; mixed 84, 99, 340, 132.  P4 with three
+// threads per column spills (96 registers): FP64 262.
+// P1's 64-thread CTAs need eight per SM in FP64 (128 registers, 184 bytes
+// spilled) where the tiles fill them; where four per SM hold every tile the
+// spills only lengthen a tile: grad_few (232 registers) 8^3 18.3 -> 17.3.
 template <typename A, int N>
 struct HexNsShape
 {
@@ -610,6 +610,7 @@ struct HexNsShape
   static constexpr int grad_zs = N == 3 ? 3 : 2;
   static constexpr int grad_minb =
       N == 2 ? (f64 ? 8 : 16) : N == 3 ? (f64 ? 2 : 4) : N == 5 ? (f64 ? 1 : 2) : (f64 ? 2 : 4);
+  static constexpr int grad_few = N == 2 && f64 ? 4 : grad_minb;
 };
 
 // Launch shape of the face kernel, by what it does.  ONE: the one-sided form,
@@ -645,8 +646,8 @@ struct HexFaceShape
 // Navier-Stokes kernel 1 (column mapping): common solution, gradient, viscous
 // normal flux at own flux points, flux, volume divergence
 // ---------------------------------------------------------------------------
-template <typename T, typename A, int N>
-__global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsShape<A, N>::grad_minb)
+template <typename T, typename A, int N, int MINB>
+__global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, MINB)
     k_hex_ns_grad(const __grid_constant__ Args<T, A> a, const __grid_constant__ LineOpsT<A, N> ops)
 {
   using H = HexIdx<N>;
@@ -667,12 +668,15 @@ __global__ void __launch_bounds__(TW * N * N * HexNsShape<A, N>::grad_zs, HexNsS
   if (tile >= a.ntiles) return;
   // the tile's metrics (gradient and flux passes) and face geometry (viscous
   // pass) on their way to L2 while the state and partner traces load; the
-  // state and codes of the tile one wave of resident CTAs ahead (2 per SM)
+  // state and codes of the tile one wave ahead of it where one or two CTAs share
+  // an SM.  Where more do, that tile is on the SM already and the request finds
+  // its lines in L2: no time lost or won (mixed P2 30^3 80.3 us with, 81.8
+  // without; FP64 P1 44^3 150.7 and 150.7).
   if (threadIdx.x == 0)
   {
     prefetch_l2(a.mets + tile * (int64_t)S * 10 * TW, S * 10 * TW * sizeof(T));
     prefetch_l2(a.fgeo + tile * (int64_t)Fp * 4 * TW, Fp * 4 * TW * sizeof(T));
-    const int64_t ahead = tile + 2 * 148;
+    const int64_t ahead = tile + 148 * (MINB < 2 ? 1 : 2);
     if (ahead < a.ntiles)
     {
       prefetch_l2(a.U + ahead * (int64_t)S * V * TW, S * V * TW * sizeof(T));

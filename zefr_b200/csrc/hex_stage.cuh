@@ -20,6 +20,19 @@ static void launch_euler_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &
   CK(cudaGetLastError());
 }
 
+template <typename T, typename A, int N, int MINB>
+static void launch_grad_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
+{
+  using G = Shape<3, N>;
+  const size_t smem = (size_t)((4 * G::S * G::V + G::Fp * G::V) * TW + 3 * N * TW) * sizeof(A);  // + sX padding
+  set_smem(dev::k_hex_ns_grad<T, A, N, MINB>, smem);
+  ProfScope ps(c, ZB_K_NS_GRAD);
+  dev::k_hex_ns_grad<T, A, N, MINB>
+      <<<(unsigned)c.ntiles, TW * N * N * dev::HexNsShape<A, N>::grad_zs, smem, c.stream>>>(a, ops);
+  c.launches++;
+  CK(cudaGetLastError());
+}
+
 template <typename T, typename A, int N, bool ONE, bool RK>
 static void launch_face_hex(Ctx &c, const Args<T, A> &a, const LineOpsT<A, N> &ops)
 {
@@ -46,12 +59,8 @@ static void launch_extrap_hex(Ctx &c)
 template <typename T, typename A, int N>
 static void launch_stage_hex(Ctx &c, const StageCfg &sc)
 {
-  using G = Shape<3, N>;
-  constexpr int S = G::S, Fp = G::Fp, V = G::V;
   const Args<T, A> a = make_args<T, A>(c, sc);
   const LineOpsT<A, N> ops = line_ops<A, N>(c.plan);
-  // hexahedra: column-mapped kernels, TW x N^2 threads per tile
-  constexpr int HT = TW * N * N;
   if (!c.plan.params.viscous)
   {
     using E = dev::HexEulerShape<A, N>;
@@ -62,15 +71,13 @@ static void launch_stage_hex(Ctx &c, const StageCfg &sc)
   }
   else
   {
-    constexpr int ZG = dev::HexNsShape<A, N>::grad_zs;
-    const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(A);  // + sX padding
-    set_smem(dev::k_hex_ns_grad<T, A, N>, smem1);
+    using G1 = dev::HexNsShape<A, N>;
     if (!sc.face_only)
     {
-      ProfScope ps(c, ZB_K_NS_GRAD);
-      dev::k_hex_ns_grad<T, A, N><<<(unsigned)c.ntiles, HT * ZG, smem1, c.stream>>>(a, ops);
-      c.launches++;
-      CK(cudaGetLastError());
+      if (c.ntiles > (int64_t)148 * G1::grad_few)
+        launch_grad_hex<T, A, N, G1::grad_minb>(c, a, ops);
+      else
+        launch_grad_hex<T, A, N, G1::grad_few>(c, a, ops);
     }
     if (sc.grad_only) return;
     if (a.Fcom)

@@ -252,11 +252,12 @@ void run_kernels(const Plan &p, unsigned char *base, const Regions &r, cudaStrea
     }
     else
     {
-      constexpr int ZG = dev::HexNsShape<double, N>::grad_zs;
+      using G1 = dev::HexNsShape<double, N>;
       const size_t smem1 = (size_t)((S * V + Fp * V + 3 * S * V) * TW + 3 * N * TW) * sizeof(double);
-      NA_CK(cudaFuncSetAttribute(dev::k_hex_ns_grad<double, double, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem1));
-      dev::k_hex_ns_grad<double, double, N><<<(unsigned)p.ntiles, HT * ZG, smem1, st>>>(a, ops);
+      auto grad = p.ntiles > (int64_t)148 * G1::grad_few ? dev::k_hex_ns_grad<double, double, N, G1::grad_minb>
+                                                         : dev::k_hex_ns_grad<double, double, N, G1::grad_few>;
+      NA_CK(cudaFuncSetAttribute(grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1));
+      grad<<<(unsigned)p.ntiles, HT * G1::grad_zs, smem1, st>>>(a, ops);
       NA_CK(cudaGetLastError());
       const size_t smem2 = (size_t)Fp * V * TW * sizeof(double);
       const auto face = [&](auto kernel, int zs) {
