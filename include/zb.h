@@ -362,7 +362,7 @@ zb_status zb_vjp_geometry(zb_ctx *ctx, const double *lam, double *Ubar, int64_t 
  * != 0 the metric adjoint of the stage residuals and of the update's 1/|J|
  * is added to the device sums zb_geometry_adjoint_get reads.  Uses the
  * context's fixed dt (zb_set_dt; ZB_ERR_UNSUPPORTED under RK54 or a CFL
- * step); leaves the context's state undefined.  No reference
+ * step); the context keeps its state and residual registers.  No reference
  * counterpart. */
 zb_status zb_rk_step_vjp(zb_ctx *ctx, const double *U0, const double *Ubar1, double *Ubar0, int64_t spt_stride,
                          int64_t var_stride, int64_t ele_stride, int where, double *param_bar, int geometry);

@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 import golden_cases as gc
-from zefr_b200.solver import FRSolver, params_from_reference
+from zefr_b200 import meshgen
+from zefr_b200.solver import FRSolver, make_params, params_from_reference
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -67,6 +68,93 @@ def test_rk_step_vjp_equals_composed_stage_adjoints(name):
     err = np.abs(got.cpu().numpy() - ref).max() / np.abs(ref).max()
     assert err <= 1e-12, err
     assert np.allclose(pbar, pref, rtol=1e-12, atol=1e-12 * np.abs(pref).max())
+
+
+# mesh, order, viscous, beta, flux, boundaries; hexahedra take the one-sided form
+# (beta = +-1/2: traces formed from the state, no trace buffer) or the trace
+# buffer (any other beta)
+STEP_CASES = {
+    "hex_euler": ("hex", 2, False, 0.5, "rusanov", "periodic"),
+    "hex_ns_b05": ("hex", 3, True, 0.5, "roe", "periodic"),
+    "hex_ns_bm05": ("hex", 2, True, -0.5, "rusanov", "periodic"),
+    "hex_ns_b025": ("hex", 2, True, 0.25, "roe", "periodic"),
+    "hex_ns_char": ("hex", 2, True, 0.5, "rusanov", "char"),
+    "hex_ns_char_b025": ("hex", 1, True, 0.25, "roe", "char"),
+    "hex_euler_char": ("hex", 2, False, 0.5, "roe", "char"),
+    "quad_ns_char": ("quad", 4, True, 0.5, "roe", "char"),
+    "quad_ns_wall": ("quad", 3, True, 0.3, "rusanov", "wall_ns_adi"),
+    "tri_ns_char": ("tri", 2, True, -0.5, "roe", "char"),
+}
+
+
+@pytest.mark.parametrize("name", list(STEP_CASES))
+def test_rk_step_vjp_with_geometry_and_kept_state(name):
+    """The step adjoint against the transpose composed here from the residual
+    adjoints, as above, with the free-stream and (quadrilaterals, hexahedra)
+    the geometry adjoint: U_s depends on |J| through a dt R / |J|, which adds
+    a_{s-1} dt Ubar_s . R_{s-1} / |J|^2 and dt b_s Ubar_1 . R_s / |J|^2 to the
+    stages' own sums.  Same kernels in a different order of sums: 1e-12
+    relative.  A state set before the call is still the context's after it."""
+    etype, order, viscous, ldg_b, flux, bc = STEP_CASES[name]
+    tag = "PERIODIC" if bc == "periodic" else "SIDE"
+    mesh = {"hex": lambda: meshgen.jitter_interior(meshgen.box_hexes(4, 3, 3, bnd=tag), 0.1, 5),
+            "quad": lambda: meshgen.jitter_interior(meshgen.box_quads(5, 4, 0.0, 1.0, 0.0, 1.0, bnd=tag), 0.02, 5),
+            "tri": lambda: meshgen.box_tris(4, jitter=0.1, bnd=tag)}[etype]()
+    dt = 1e-3
+    s = FRSolver(mesh, make_params(order, viscous, gamma=1.4, prandtl=0.71, mu=2e-3, ldg_b=ldg_b, ldg_tau=0.1,
+                                   fconv=flux, V_fs=(0.3, 0.1, 0.0), dt=dt), {tag: bc})
+    S, V, E = s.state_shape
+    rng = np.random.default_rng(3)
+    U0 = 0.05 * rng.standard_normal(s.state_shape)
+    U0[:, 0] += 1.0
+    U0[:, 1] += 0.2
+    U0[:, -1] += 2.6
+    U0, ub = torch.from_numpy(U0).cuda(), torch.from_numpy(rng.standard_normal(s.state_shape)).cuda()
+    det = torch.from_numpy(s.plan.get("jaco_det_spts").reshape(S, 1, E)).cuda()
+    geo = etype != "tri"
+    alpha, beta = (0.5, 0.5, 1.0), (1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0)
+    Us, Rs = [U0], []
+    for st in range(4):
+        s.set_state(Us[st])
+        s.compute_residual(0)
+        R = torch.empty_like(U0)
+        s.get_residual_device(R, 0)
+        Rs.append(R)
+        if st < 3:
+            Us.append(U0 - alpha[st] * dt / det * R)
+    ub0, ub_next, pref, det_bar = ub.clone(), None, np.zeros(5), torch.zeros((S, E), dtype=torch.float64, device="cuda")
+    for st in range(3, -1, -1):
+        lam = -beta[st] * dt / det * ub
+        if ub_next is not None:
+            lam = lam - alpha[st] * dt / det * ub_next
+        s.set_state(Us[st])
+        ub_next, p = s.vjp_geometry_accumulate(lam) if geo else s.vjp(lam.contiguous(), params=True)
+        pref += p
+        ub0 = ub0 + ub_next
+        if st > 0:
+            det_bar += (alpha[st - 1] * dt * ub_next * Rs[st - 1] / det ** 2).sum(1)
+        det_bar += (beta[st] * dt * ub * Rs[st] / det ** 2).sum(1)
+    if geo:
+        want = s.geometry_adjoint()
+        want["jaco_det"] = want["jaco_det"] + det_bar.cpu().numpy()
+    # the call itself, with another state in the context
+    A = U0 * 1.01
+    s.set_state(A)
+    s.compute_residual(1)
+    R1, U1 = s.get_residual(1), s.get_state()
+    pbar = np.zeros(5)
+    got = s.rk_step_vjp(U0, ub, pbar, geometry=geo)
+    ref = ub0.cpu().numpy()
+    assert np.abs(got.cpu().numpy() - ref).max() <= 1e-12 * np.abs(ref).max()
+    assert np.allclose(pbar, pref, rtol=1e-12, atol=1e-12 * max(np.abs(pref).max(), 1e-300))
+    assert (np.abs(pbar).max() > 0) == (bc == "char")
+    if geo:
+        for k, v in s.geometry_adjoint().items():
+            assert np.abs(v - want[k]).max() <= 1e-12 * np.abs(want[k]).max(), k
+    assert np.array_equal(s.get_state(), U1) and np.array_equal(s.get_residual(1), R1)
+    s.compute_residual(0)
+    assert np.array_equal(s.get_residual(0), R1)
+    s.close()
 
 
 def _fd_objective(traj, U0, v, h, nsteps, obj):
