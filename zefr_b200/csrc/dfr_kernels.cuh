@@ -1,5 +1,7 @@
-// Tensor-product DFR residual kernels for quadrilaterals (D = 2) and
-// hexahedra (D = 3) of order P = N - 1, templated on the arithmetic type.
+// What the residual kernels share, templated on the arithmetic type: the tile
+// layout, the line operators of quadrilaterals (D = 2) and hexahedra (D = 3) of
+// order P = N - 1, the 2D faces and the RK update of a point.  The kernels are in
+// quad_kernels.cuh, hex_kernels.cuh and tri_kernels.cuh.
 //
 // Data layout in HBM is tile-major structure-of-arrays: TW consecutive
 // elements form a tile and every per-element array is stored as
@@ -168,12 +170,6 @@ __device__ __forceinline__ void load_ops(A *sops, const LineOpsT<A, N> &ops, int
   const A *src = reinterpret_cast<const A *>(&ops);
   constexpr int n = N * N + 4 * N;
   for (int i = tid; i < n; i += nth) sops[i] = src[i];
-}
-
-template <typename A, int N>
-__device__ __forceinline__ void load_ops(A *sops, const LineOpsT<A, N> &ops)
-{
-  load_ops<A, N>(sops, ops, threadIdx.x, blockDim.x);
 }
 
 // Barrier of the threads running one tile: the whole block (bar == 0) or a

@@ -20,7 +20,6 @@ struct TriShape
   static constexpr int D = 2, V = 4, NM = 5;
   static constexpr int S = N * (N + 1) / 2;
   static constexpr int Fp = 3 * N;
-  static constexpr int NT = 128;
   // dense operator block: oppE [Fp][S], oppD [D][S][S], oppD_fpts [D][S][Fp],
   // oppDiv [S][D*S], oppDiv_fpts [S][Fp]
   static constexpr int OE = 0, OD = OE + Fp * S, ODF = OD + D * S * S, ODV = ODF + D * S * Fp,
@@ -74,13 +73,16 @@ __device__ __forceinline__ void tri_transform(const A F[4][2], const A adj[2][2]
 // shared memory once per CTA and not once per tile (all five, at P4 14 KB in
 // FP64 beside 4 KB of state per tile; P8 104 KB).  minb: CTAs per SM the
 // registers and the shared memory allow, as resident threads.  Against one
-// 128-thread CTA per tile, us, Navier-Stokes Roe gradient / face with RK
-// update and Euler Rusanov, 2 x 110^2 elements (P6, P8: 2 x 60^2):
-//   FP64  P1 23 -> 15 / 32 -> 18, 30 -> 16;  P3 36 -> 34 / 41 -> 31, 43 -> 32;
-//         P5 112 -> 97 / 86 -> 66, 101 -> 85;  P8 224 -> 111 / 113 -> 51, 142 -> 85
-//   mixed P1 15 -> 13 / 15.5 -> 13, 14 -> 12;  P3 23 -> 23 / 21 -> 20, 22 -> 22;
-//         P5 53 -> 53 / 38 -> 38, 47 -> 45;  P8 82 -> 61 / 46 -> 29, 62 -> 47
-// FP64 face at 512 threads spills the update's inputs: P3 35.
+// 128-thread CTA per tile (with whole flux matrices per face point), us,
+// Navier-Stokes Roe gradient / face with RK update and Euler Roe with RK update,
+// 2 x 110^2 elements (P8: 2 x 60^2):
+//   FP64  P1 31 -> 15 / 35 -> 18, 31 -> 17;  P3 47 -> 32 / 44 -> 30, 46 -> 32;
+//         P5 108 -> 93 / 90 -> 65, 111 -> 85;  P8 248 -> 107 / 123 -> 51, 165 -> 83
+//   mixed P1 16 -> 12 / 17 -> 13, 17 -> 13;  P3 25 -> 21 / 22 -> 20, 25 -> 22;
+//         P5 59 -> 51 / 39 -> 38, 50 -> 43;  P8 73 -> 56 / 46 -> 28, 68 -> 44
+// The FP64 face kernel's 400 threads (168 registers) spill 130-160 bytes at most
+// orders; 256 threads (222 registers) spill none and take longer: P1 17.9 -> 21.3,
+// P3 30.4 -> 38.9, P5 65 -> 94.
 template <typename A, int N>
 struct TriRun
 {
