@@ -1359,12 +1359,12 @@ __global__ void __launch_bounds__(Shape<D, N>::NT, adj_ns1_minb<D, N, GEO>()) k_
   const int64_t tile = blockIdx.x;
   if (tile >= a.ntiles) return;
   // this tile's metrics (gradient, volume and gradient-adjoint passes) and
-  // the inputs of the tile one wave of resident CTAs (one per SM) ahead on
-  // their way to L2
+  // the inputs of the tile one wave of resident CTAs ahead on their way to L2
+  // (without it P4 quadrilaterals, 140^2 Roe, 122 -> 127 us)
   if (threadIdx.x == 0)
   {
     prefetch_l2(a.mets + tile * (int64_t)S * NM * TW, S * NM * TW * sizeof(double));
-    const int64_t ahead = tile + 148;
+    const int64_t ahead = tile + 148 * adj_ns1_minb<D, N, GEO>();
     if (ahead < a.ntiles)
     {
       prefetch_l2(a.Ufp + ahead * (int64_t)Fp * V * TW, Fp * V * TW * sizeof(double));
