@@ -84,9 +84,10 @@ def test_many_tiles_repeat_the_few(kind, n):
 # GPU holds CTAs of any triangle kernel of that order and form (148 SMs times
 # the most CTAs per SM: 20, 13, 13, 3 of the FP32 gradient and Euler kernels at
 # P1, P2, P3, P8, 16, 16, 4 of the extrapolation from P2 on; FP64 8, 5, 5, 1):
-# every CTA walks on to another tile, in FP64 to several.  At P2 this is also
-# where the extrapolation takes its other form.
-MANY = [("fp64", 1, 125), ("fp64", 2, 100), ("mixed", 2, 100), ("fp64", 3, 100), ("fp64", 8, 45), ("mixed", 1, 125), ("mixed", 3, 105), ("mixed", 8, 52)]
+# every CTA walks on to another tile, in FP64 to several.  P1 n 125 and P2 n 184
+# are also where the extrapolation takes its form for large meshes.
+MANY = [("fp64", 1, 125), ("fp64", 2, 100), ("mixed", 2, 100), ("fp64", 2, 184), ("mixed", 2, 184),
+        ("fp64", 3, 100), ("fp64", 8, 45), ("mixed", 1, 125), ("mixed", 3, 105), ("mixed", 8, 52)]
 
 
 @pytest.mark.parametrize("viscous,beta,fconv", [(False, 0.5, "roe"), (True, 0.5, "rusanov"), (True, 0.3, "roe")])

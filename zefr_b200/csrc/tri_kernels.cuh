@@ -219,14 +219,15 @@ __global__ void __launch_bounds__(128) k_tri_extrap_direct(const T *__restrict__
 // The same with the tile's state in shared memory: a flux point reads S 16-byte
 // groups there instead of 4 S values, for two barriers per tile.  us, 2 n^2
 // triangles, direct -> this form, FP64 and mixed: P4 n 110 18.6 -> 14.6 and 12.7
-// -> 10.8, P3 n 110 12.6 -> 10.5 and 10.1 -> 8.7.  At P1 a tile's 48 traces are
-// less work than the barriers (n 110 7.6 -> 8.5 and 6.7 -> 8.3, n 300 14.2 ->
-// 15.8 and 11.5 -> 13.7), and at P2 where CTAs take more than one tile (n 60
-// 8.6 -> 6.8 and 6.9 -> 6.4, n 110 equal, n 300 24.9 -> 26.9 and 17.2 -> 19.4).
+// -> 10.8, P3 n 110 12.6 -> 10.5 and 10.1 -> 8.7, P2 n 60 8.6 -> 6.6 and 7.0 ->
+// 6.6, n 130 the same.  On large meshes the barriers outweigh the little work per
+// tile: at P1 past 14 tiles per SM (n 90 the same, n 110 7.3 -> 8.6 and 6.6 ->
+// 8.6, n 300 13.1 -> 16.0 and 11.6 -> 13.7), at P2 past 56 (n 160 12.7 -> 11.7 and
+// 10.1 -> 10.2, n 300 24.9 -> 26.9 and 17.2 -> 19.4).
 template <int N>
-constexpr bool tri_extrap_direct(int64_t ntiles, int64_t resident_ctas)
+constexpr bool tri_extrap_direct(int64_t ntiles)
 {
-  return N == 2 || (N == 3 && ntiles > resident_ctas);
+  return (N == 2 && ntiles > 148 * 14) || (N == 3 && ntiles > 148 * 56);
 }
 
 template <typename T, typename A, int N>

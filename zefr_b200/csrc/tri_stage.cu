@@ -10,23 +10,22 @@ template <typename T, typename A, int N>
 static void launch_extrap_tri(Ctx &c)
 {
   using R = dev::TriRun<A, N>;
-  const int64_t resident = (int64_t)148 * R::extrap_minb;
   const T *U = (const T *)c.U;
   T *Ufp = (T *)c.Ufp[c.cur];
   const A *ops = (const A *)c.dops;
   ProfScope ps(c, ZB_K_EXTRAP);
-  const bool direct = dev::tri_extrap_direct<N>(c.ntiles, resident);
-  if constexpr (N <= 3)
-    if (direct)
+  if (dev::tri_extrap_direct<N>(c.ntiles))
+  {
+    if constexpr (N <= 3)
       dev::k_tri_extrap_direct<T, A, N>
           <<<grid_for(c.ntiles * dev::TriShape<N>::Fp * TW, 128), 128, 0, c.stream>>>(U, Ufp, c.ntiles, ops);
-  if constexpr (N > 2)
-    if (!direct)
-    {
-      set_smem(dev::k_tri_extrap<T, A, N>, R::extrap_smem);
-      dev::k_tri_extrap<T, A, N>
-          <<<(unsigned)std::min(c.ntiles, resident), R::NT, R::extrap_smem, c.stream>>>(U, Ufp, c.ntiles, ops);
-    }
+  }
+  else
+  {
+    set_smem(dev::k_tri_extrap<T, A, N>, R::extrap_smem);
+    const unsigned grid = (unsigned)std::min<int64_t>(c.ntiles, (int64_t)148 * R::extrap_minb);
+    dev::k_tri_extrap<T, A, N><<<grid, R::NT, R::extrap_smem, c.stream>>>(U, Ufp, c.ntiles, ops);
+  }
   c.launches++;
   CK(cudaGetLastError());
 }
